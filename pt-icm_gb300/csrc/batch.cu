@@ -78,7 +78,8 @@ struct pticm_batch {
     DArr<int32_t> d_sched_off, d_sched, d_rep_inst, d_row, d_col, d_h;
     DArr<uint32_t> d_adj, d_thr, d_slot, d_order;
     DArr<double> d_beta;
-    DArr<int8_t> d_spins, d_pub, d_best_state;
+    DArr<int8_t> d_spins, d_best_state;
+    DArr<unsigned long long> d_pub;   // published spin words (two halves)
     DArr<int32_t> d_fields;
     DArr<long long> d_E, d_Epub, d_bestE;
     DArr<unsigned long long> d_flips, d_bestSweep, d_att, d_succ, d_mismatch, d_job_ns;
@@ -289,7 +290,7 @@ EngineArgs batch_args(pticm_batch* b) {
     A.fields = b->d_fields.p;
     A.energy = b->d_E.p;
     A.spins_pub = b->d_pub.p;
-    A.spins_pub_half = (long long)b->d_spins.n;
+    A.spins_pub_half = (long long)b->d_spins.n / 16;
     A.energy_pub = b->d_Epub.p;
     A.energy_pub_half = (long long)b->d_E.n;
     A.flips = b->d_flips.p;
@@ -307,6 +308,7 @@ EngineArgs batch_args(pticm_batch* b) {
         for (const HostProblem& P : b->P) b->ebound = std::max(b->ebound, energy_bound(P));
     }
     A.flag_barrier = b->ebound < (1ll << 31) ? 1 : 0;   // every energy fits the word's 32 bits
+    A.small_energy = b->ebound < (1ll << 30) ? 1 : 0;
     A.abort_flag = b->d_abort.p;
     A.status = b->d_status.p;
     A.sweeps = (int)b->o.sweeps;
@@ -501,7 +503,7 @@ int pticm_batch_create(const pticm_problem* const* problems, uint32_t count, con
     BCK(b->d_spins.alloc(spin_total));
     BCK(b->d_fields.alloc(spin_total));
     BCK(b->d_best_state.alloc(spin_total));
-    BCK(b->d_pub.alloc(2 * spin_total));
+    BCK(b->d_pub.alloc(2 * (spin_total / 16)));
     BCK(b->d_E.alloc(rep_total));
     BCK(b->d_Epub.alloc(2 * rep_total * kPubStride));
     BCK(b->d_bestE.alloc(rep_total));

@@ -206,6 +206,9 @@ extern "C" int pticm_run_noalloc(const pticm_problem* p, const pticm_opts* o, co
     NA_CK(cudaMemsetAsync(base + o_bestS, 0, RR * 8, st));
     NA_CK(cudaMemsetAsync(base + o_att, 0, RR * 8, st));
     NA_CK(cudaMemsetAsync(base + o_succ, 0, RR * 8, st));
+    // (words left there by another run could carry any tag)
+    NA_CK(cudaMemsetAsync(base + o_pub, 0, RR * npad, st));
+    NA_CK(cudaMemsetAsync(base + o_Epub, 0, 2 * RR * 8 * kPubStride, st));
     if (io->slot_to_replica)
         NA_CK(cudaMemcpyAsync(base + o_slot, io->slot_to_replica, RR * 4, cudaMemcpyDeviceToDevice, st));
     else
@@ -252,8 +255,8 @@ extern "C" int pticm_run_noalloc(const pticm_problem* p, const pticm_opts* o, co
     A.spins = reinterpret_cast<int8_t*>(base + o_spins);
     A.fields = reinterpret_cast<int32_t*>(base + o_fields);
     A.energy = reinterpret_cast<long long*>(base + o_E);
-    A.spins_pub = reinterpret_cast<int8_t*>(base + o_pub);
-    A.spins_pub_half = (long long)RR * npad;
+    A.spins_pub = reinterpret_cast<unsigned long long*>(base + o_pub);
+    A.spins_pub_half = (long long)(RR * npad / 16);
     A.energy_pub = reinterpret_cast<long long*>(base + o_Epub);
     A.energy_pub_half = R;
     A.flips = reinterpret_cast<unsigned long long*>(base + o_flips);
@@ -267,6 +270,7 @@ extern "C" int pticm_run_noalloc(const pticm_problem* p, const pticm_opts* o, co
     A.successes = reinterpret_cast<unsigned long long*>(base + o_succ);
     A.bar = reinterpret_cast<unsigned int*>(base + o_bar);
     A.flag_barrier = energy_bound(P) < (1ll << 31) ? 1 : 0;   // every energy fits the word's 32 bits
+    A.small_energy = energy_bound(P) < (1ll << 30) ? 1 : 0;
     A.abort_flag = reinterpret_cast<int*>(base + o_abort);
     A.status = reinterpret_cast<DevStatus*>(base + o_status);
     A.sweeps = (int)o->sweeps;

@@ -36,23 +36,26 @@ __device__ __forceinline__ T* sm_ptr(uint8_t* base, uint32_t off) {
     return reinterpret_cast<T*>(base + off);
 }
 
-// Thread-0 phase timers (clock64), enabled by EngineArgs::prof.
+// Thread-0 phase timers (clock64), enabled by EngineArgs::prof; the marks and
+// counters live in shared memory, so that an unprofiled run keeps nothing of
+// them in registers.
+struct ProfStore {
+    long long mark, sub;
+    long long c[PROF_PHASES];
+};
 struct Prof {
     bool on;
-    long long mark, sub;
-    long long* c;   // PROF_PHASES counters in shared memory (thread 0 only)
-    __device__ __forceinline__ void init(bool enable, long long* store) {
-        on = enable;
-        c = store;
-        mark = sub = enable ? clock64() : 0;
-        if (enable)
-            for (int q = 0; q < PROF_PHASES; q++) c[q] = 0;
+    ProfStore* s;
+    __device__ __forceinline__ void init() const {
+        if (!on) return;
+        s->mark = s->sub = clock64();
+        for (int q = 0; q < PROF_PHASES; q++) s->c[q] = 0;
     }
-    __device__ __forceinline__ void tick(int slot) {
-        if (on) { const long long t = clock64(); c[slot] += t - mark; mark = t; sub = t; }
+    __device__ __forceinline__ void tick(int slot) const {
+        if (on) { const long long t = clock64(); s->c[slot] += t - s->mark; s->mark = t; s->sub = t; }
     }
-    __device__ __forceinline__ void subtick(int slot) {
-        if (on) { const long long t = clock64(); c[slot] += t - sub; sub = t; }
+    __device__ __forceinline__ void subtick(int slot) const {
+        if (on) { const long long t = clock64(); s->c[slot] += t - s->sub; s->sub = t; }
     }
 };
 
@@ -87,54 +90,86 @@ __device__ __forceinline__ bool uf_unite(int* parent, int a, int b) {
 
 // ---------------------------------------------------------- team helpers
 // An ICM "team" is either one warp (many pairs per block) or the whole block
-// (one pair per block).  Block-wide reductions go through shared scratch.
-// A block team reduces through three slots of four words, used in turn: a
-// slot is reset by the reduction after the one that used it (whose barrier
-// every reader of the slot has passed), so one barrier per reduction
-// suffices.  Between teams all slots hold the identity (0, ~0, ~0, 0).
-__device__ __forceinline__ void team_slot_reset(long long* acc, int slot) {
-    unsigned long long* u = reinterpret_cast<unsigned long long*>(acc) + 4 * slot;
-    u[0] = 0;
-    u[1] = ~0ull;
-    u[2] = ~0ull;
-    u[3] = 0;
+// (one pair per block).  A warp reduces with redux instructions; the warps of
+// a block team meet in shared memory, with one barrier per reduction: keys in
+// a slot per warp, sums by one 32-bit atomic per warp (64-bit shared atomic
+// minima are compare-and-swap loops: sixteen warps queueing on them took
+// 0.5 us per reduction).
+__device__ __forceinline__ unsigned long long warp_min(unsigned long long k) {
+    const uint32_t hi = __reduce_min_sync(0xffffffffu, (uint32_t)(k >> 32));
+    const uint32_t lo = __reduce_min_sync(0xffffffffu, (uint32_t)(k >> 32) == hi ? (uint32_t)k : 0xFFFFFFFFu);
+    return ((unsigned long long)hi << 32) | lo;
 }
+
+// Control words of a team in shared memory (a warp team uses the first two).
+enum TeamCtl : int {
+    TC_BEST = 0,      // warp team: the giant component's root
+    TC_TAIL = 1,      // breadth-first queue tail
+    TC_OVERLAP = 2,   // overlap sites listed, zero between pairs
+    TC_OTHERS = 3,    // other sites listed, zero between pairs
+    TC_S = 4,         // sites listed outside the giant component, zero between pairs
+    TC_STALE = 5,     // a published word had not arrived, zero between pairs
+    TC_COUNT = 6,     // a sum of counts; zeroed when a pair begins
+    TC_DE = 8,        // two 64-bit energy changes; zeroed when a pair begins
+    TC_WORDS = 16
+};
 
 template <bool BLOCK>
 struct Team {
     int tr, ts;                  // rank and size
-    long long* acc;              // team scratch (shared, 12 words for a block team)
-    int* ctl;                    // team scratch (shared): BFS queue tail, vote
-    mutable int k = 0;           // reductions so far (the same in every thread)
+    int* ctl;                    // control words (shared)
+    unsigned long long* keys;    // block team: two keys per warp (shared)
     __device__ __forceinline__ void sync() const {
         if (BLOCK) __syncthreads(); else __syncwarp();
     }
-    // (sum, min, min, sum) over the team
-    __device__ __forceinline__ void reduce(long long& s0, unsigned long long& m1, unsigned long long& m2,
-                                           long long& s3) const {
+    // A pair begins.  The sums' readers of the pair before have passed a
+    // barrier since, and one comes before the next use.
+    __device__ __forceinline__ void begin() const {
+        if (BLOCK && tr == 0) {
+            ctl[TC_COUNT] = 0;
+            reinterpret_cast<unsigned long long*>(ctl + TC_DE)[0] = 0ull;
+            reinterpret_cast<unsigned long long*>(ctl + TC_DE)[1] = 0ull;
+        }
+    }
+    // Sum of a count over the team, once per pair.
+    __device__ __forceinline__ int count(int c) const {
+        c = __reduce_add_sync(0xffffffffu, c);
+        if (!BLOCK) return c;
+        if ((threadIdx.x & 31) == 0 && c != 0) atomicAdd(ctl + TC_COUNT, c);
+        __syncthreads();
+        return *(volatile int*)(ctl + TC_COUNT);
+    }
+    // Sums of two energy changes, for the thread of rank 0, once per pair.
+    // With `small` (all energies within 2^30) both are exact modulo 2^32.
+    __device__ __forceinline__ void sum_energies(long long& a, long long& b, bool small) const {
+        unsigned long long* const acc = reinterpret_cast<unsigned long long*>(ctl + TC_DE);
+        if (small) {
+            int x = (int)__reduce_add_sync(0xffffffffu, (unsigned)a), y = (int)__reduce_add_sync(0xffffffffu, (unsigned)b);
+            if (BLOCK) {
+                if ((threadIdx.x & 31) == 0) {
+                    if (x) atomicAdd(reinterpret_cast<int*>(acc), x);
+                    if (y) atomicAdd(reinterpret_cast<int*>(acc + 1), y);
+                }
+                __syncthreads();
+                x = *(volatile int*)acc;
+                y = *(volatile int*)(acc + 1);
+            }
+            a = x;
+            b = y;
+            return;
+        }
         for (int o = 16; o > 0; o >>= 1) {
-            s0 += __shfl_xor_sync(0xffffffffu, s0, o);
-            m1 = min(m1, __shfl_xor_sync(0xffffffffu, m1, o));
-            m2 = min(m2, __shfl_xor_sync(0xffffffffu, m2, o));
-            s3 += __shfl_xor_sync(0xffffffffu, s3, o);
+            a += __shfl_xor_sync(0xffffffffu, a, o);
+            b += __shfl_xor_sync(0xffffffffu, b, o);
         }
         if (!BLOCK) return;
-        const int slot = k % 3;
-        unsigned long long* u = reinterpret_cast<unsigned long long*>(acc) + 4 * slot;
         if ((threadIdx.x & 31) == 0) {
-            atomicAdd(u + 0, (unsigned long long)s0);
-            atomicMin(u + 1, m1);
-            atomicMin(u + 2, m2);
-            atomicAdd(u + 3, (unsigned long long)s3);
+            atomicAdd(acc, (unsigned long long)a);
+            atomicAdd(acc + 1, (unsigned long long)b);
         }
         __syncthreads();
-        s0 = (long long)u[0]; m1 = u[1]; m2 = u[2]; s3 = (long long)u[3];
-        if (threadIdx.x == 0 && k > 0) team_slot_reset(acc, (k + 2) % 3);
-        k++;
-    }
-    __device__ __forceinline__ void sum2(long long& a, long long& b) const {
-        unsigned long long x = ~0ull, y = ~0ull;
-        reduce(a, x, y, b);
+        a = (long long)*(volatile unsigned long long*)acc;
+        b = (long long)*(volatile unsigned long long*)(acc + 1);
     }
 };
 
@@ -146,15 +181,37 @@ __device__ __forceinline__ unsigned long long mix64(unsigned long long z) {
     return z ^ (z >> 31);
 }
 
-// Per-block view of the launch.
+// Where a launch's data lives, known at compile time, so that the pointers
+// below have a known address space: a shared load or atomic through a
+// generic pointer first finds out where it points (on the N=2000 workload
+// the sweep, the cluster search and the flips all shorten by a tenth).
+enum Space : int {
+    SP_ANY = 0,      // found out at run time
+    SP_SHARED = 1,   // adjacency staged; replicas, thresholds and cluster scratch in shared memory
+    SP_STATE = 2,    // as SP_SHARED, but the adjacency may be in device memory (an instance of a batch)
+    SP_LARGE = 3,    // spins and cluster scratch in shared memory; adjacency, thresholds and the overlap list in device memory
+};
+
+// The cluster search unites along every edge, instead of sampling links first,
+// for few neighbours, few colour classes (two or three: the sites of one class
+// all hook under sites of the others, so the trees stay shallow) and few sites
+// per thread: on the +-1 lattice of 400 sites the search takes 3.3 us against
+// 5.6 (step 15.3 -> 12.7 us), of 1764 sites the step 1.2 times less; with mean
+// degree 8 it takes 5.5 against 4.8, and on a random graph of 15515 sites and
+// degree 4.7 the unions' walks to the giant component's root made the step
+// 2.8 times longer.
+constexpr int kDirectDegree = 5, kDirectSites = 2560;
+
+// Per-block view of a job: its descriptor (in shared memory) and pointers,
+// which are shared-memory offsets of the launch's plan or device addresses.
 struct BlockCtx {
-    InstanceDesc D;
+    const InstanceDesc& D;
     int rank, r0;
     const int32_t* row;
     const uint32_t* adj;
     int8_t* spin;
-    int32_t* field;
-    const int32_t* h;
+    int32_t* field;     // null: fields are gathered
+    const int32_t* h;   // null: no linear terms
     long long* E;
     uint32_t* slot;
     uint32_t* rslot;
@@ -220,23 +277,39 @@ __device__ __forceinline__ void for_each_neighbour(const int32_t* row, const uin
 // the set (s_v equal in A and B), an exact integer update.  Members held by
 // another block are read from the published copy and flipped by their own
 // block, which finds the same set.
-template <bool BLOCK, bool REPLAY, bool LS, bool GLINK = false>
-__device__ int icm_pair(const EngineArgs& A, const BlockCtx& B, const Team<BLOCK>& team, int q,
-                         int rA, int rB, unsigned long long step, int ls, const IcmScratch& X,
-                         int where_err, Prof& P) {
+template <bool BLOCK, bool REPLAY, bool LS, int SPACE, bool GLINK = false>
+__device__ __forceinline__ int icm_pair(const EngineArgs& A, const BlockCtx& B, const Team<BLOCK>& team, int q,
+                                        int rA, int rB, unsigned long long step, int ls, const IcmScratch& X,
+                                        int where_err, const Prof P) {
     const InstanceDesc& D = B.D;
     const int n = D.n, npad = D.n_pad;
-    // the block context lives in shared memory: its pointers and flags are
-    // read once here, not at every use inside the passes' loops
     const int32_t* const brow = B.row;
     const uint32_t* const badj = B.adj;
-    const int32_t* const bh = D.has_h ? B.h : nullptr;
+    const int32_t* const bh = B.h;
     const bool has_h = bh != nullptr;
     const bool locA = rA >= B.r0 && rA < B.r0 + D.rpc;
     const bool locB = rB >= B.r0 && rB < B.r0 + D.rpc;
     const int parity = (int)(step & 1ull);
-    const int8_t* pubA = A.spins_pub + parity * A.spins_pub_half + D.spin_off + (long long)rA * npad;
-    const int8_t* pubB = A.spins_pub + parity * A.spins_pub_half + D.spin_off + (long long)rB * npad;
+    // a member held by another block: its published words of this step
+    const unsigned long long* const pub0 = A.spins_pub + parity * A.spins_pub_half + (D.spin_off >> 4);
+    const unsigned long long* const pubA = pub0 + (long long)rA * (npad >> 4);
+    const unsigned long long* const pubB = pub0 + (long long)rB * (npad >> 4);
+    const uint32_t tag = A.pub_base + (uint32_t)ls;
+    // (a word that does not carry the tag yet marks the pass stale, and the
+    // pass is made again)
+    bool stale = false;
+    auto pub_bits = [&](unsigned long long w) -> uint32_t {
+        stale |= (uint32_t)(w >> 32) != tag;
+        return (uint32_t)w;
+    };
+    // sites 4 w .. 4 w + 3 of a loaded word as +-1 bytes, and one site
+    auto quad_bytes = [&](unsigned long long word, int w) -> uint32_t {
+        const uint32_t b = (pub_bits(word) >> ((w & 7) * 4)) & 15u;
+        return ~(((b * 0x00204081u) & 0x01010101u) * 0xFEu);   // bit set: 0x01, clear: 0xFF
+    };
+    auto pub_site = [&](const unsigned long long* pub, int i) -> int8_t {
+        return ((pub_bits(ld_relaxed_gpu_u64(pub + (i >> 5))) >> (i & 31)) & 1u) ? (int8_t)1 : (int8_t)-1;
+    };
     int8_t* sA = locA ? B.spin + (rA - B.r0) * npad : nullptr;
     int8_t* sB = locB ? B.spin + (rB - B.r0) * npad : nullptr;
     // no stored fields in field_gather mode: field updates are skipped
@@ -244,7 +317,7 @@ __device__ int icm_pair(const EngineArgs& A, const BlockCtx& B, const Team<BLOCK
     int32_t* fB = (locB && B.field) ? B.field + (rB - B.r0) * npad : nullptr;
     uint8_t* d = X.d;
     const int nwords = (n + 31) >> 5;
-    if (threadIdx.x == 0) P.subtick(PROF_ICM_ENERGY);
+    P.subtick(PROF_ICM_ENERGY);
     // a caller's seed for this pair (device numbering), or skip the pair
     int forced = -1;
     const bool exact = REPLAY || A.icm_exact != 0;
@@ -265,34 +338,35 @@ __device__ int icm_pair(const EngineArgs& A, const BlockCtx& B, const Team<BLOCK
                                                    (uint32_t)(step >> 32)), stream_key(A.seed, STREAM_ICM));
         r64 = ((unsigned long long)rnd.y << 32) | rnd.x;
     }
-    long long cnt = 0, hs = 0;
+    int cnt = 0;
     unsigned long long kd = ~0ull, ke = ~0ull;
+    team.begin();
     const int algo = D.icm_algo;
     auto overlap_site = [&](int i, int8_t a, int8_t b) {
         const bool di = a != b;
         d[i] = di;
         if (algo == ENGINE_ICM_UNION_FIND) X.queue[i] = i;   // union-find parents
-        cnt += di;
+        if (!BLOCK) cnt += di;
         if (!REPLAY) {
             const unsigned long long key = (mix64(r64 + 0x9E3779B97F4A7C15ull * (unsigned long long)(i + 1)) &
                                             0xFFFFFFFF00000000ull) | (unsigned)i;
             if (di) kd = min(kd, key);
             else ke = min(ke, key);
         }
-        if (has_h && locA) hs += (long long)bh[i] * a;
     };
     // a block team lists the overlap sites (from the front) and the others
     // (from the back), so that its later passes visit overlap sites only;
-    // the counters are team.ctl[2..3], zero between pairs
+    // the counters are zero between pairs
     int* lst = X.list;
+    for (unsigned int tries = 0;; tries++) {
     auto append = [&](bool valid, bool di, int i) {
         const int lane = threadIdx.x & 31;
         const unsigned mf = __ballot_sync(0xffffffffu, valid && di);
         const unsigned mb = __ballot_sync(0xffffffffu, valid && !di);
         int f0 = 0, b0 = 0;
         if (lane == 0) {
-            if (mf) f0 = atomicAdd(team.ctl + 2, __popc(mf));
-            if (mb) b0 = atomicAdd(team.ctl + 3, __popc(mb));
+            if (mf) f0 = atomicAdd(team.ctl + TC_OVERLAP, __popc(mf));
+            if (mb) b0 = atomicAdd(team.ctl + TC_OTHERS, __popc(mb));
         }
         f0 = __shfl_sync(0xffffffffu, f0, 0);
         b0 = __shfl_sync(0xffffffffu, b0, 0);
@@ -303,28 +377,29 @@ __device__ int icm_pair(const EngineArgs& A, const BlockCtx& B, const Team<BLOCK
     };
     if (BLOCK && LS) {
         // four sites per thread: one 32-bit word of each replica's spins (the
-        // partner's from the published copy in L2, one load for all four),
-        // the overlap flags stored as one word, and the sites appended to
+        // partner's expanded from its published bits, which eight threads
+        // share one L2 load of), the overlap flags stored as one word, and the sites appended to
         // the list with one warp scan and one atomic per warp and list
         // (rows are n_pad bytes, a multiple of 16: every word is aligned)
         const int lane = threadIdx.x & 31;
         const int nq = (n + 3) >> 2;
         // the next round's words are loaded before this round's are used
-        // (a partner's words come from its published copy in L2)
-        auto load_words = [&](int w, uint32_t& wa, uint32_t& wb) {
-            wa = locA ? reinterpret_cast<const uint32_t*>(sA)[w] : __ldcg(reinterpret_cast<const unsigned int*>(pubA) + w);
-            wb = locB ? reinterpret_cast<const uint32_t*>(sB)[w] : __ldcg(reinterpret_cast<const unsigned int*>(pubB) + w);
+        // (a partner's words come from L2)
+        auto load_words = [&](int w, unsigned long long& wa, unsigned long long& wb) {
+            wa = locA ? reinterpret_cast<const uint32_t*>(sA)[w] : ld_relaxed_gpu_u64(pubA + (w >> 3));
+            wb = locB ? reinterpret_cast<const uint32_t*>(sB)[w] : ld_relaxed_gpu_u64(pubB + (w >> 3));
         };
-        uint32_t na = 0, nb = 0;
+        unsigned long long na = 0, nb = 0;
         if (team.tr < nq) load_words(team.tr, na, nb);
         for (int w0 = 0; w0 < nq; w0 += team.ts) {
             const int w = w0 + team.tr;
             const bool have = w < nq;
-            const uint32_t wa = na, wb = nb;
+            const unsigned long long ra = na, rb = nb;
             if (w + team.ts < nq) load_words(w + team.ts, na, nb);
             uint32_t dw = 0;
             int fm = 0, bm = 0;
             if (have) {
+                const uint32_t wa = locA ? (uint32_t)ra : quad_bytes(ra, w), wb = locB ? (uint32_t)rb : quad_bytes(rb, w);
 #pragma unroll
                 for (int j = 0; j < 4; j++) {
                     const int i = 4 * w + j;
@@ -334,13 +409,11 @@ __device__ int icm_pair(const EngineArgs& A, const BlockCtx& B, const Team<BLOCK
                     dw |= (uint32_t)di << (8 * j);
                     fm |= (int)di << j;
                     bm |= (int)!di << j;
-                    cnt += di;
                     const unsigned long long key =
                         (mix64(r64 + 0x9E3779B97F4A7C15ull * (unsigned long long)(i + 1)) & 0xFFFFFFFF00000000ull) |
                         (unsigned)i;
                     if (di) kd = min(kd, key);
                     else ke = min(ke, key);
-                    if (has_h && locA) hs += (long long)bh[i] * a;
                 }
                 reinterpret_cast<uint32_t*>(d)[w] = dw;
                 if (algo == ENGINE_ICM_UNION_FIND)   // union-find parents
@@ -356,8 +429,8 @@ __device__ int icm_pair(const EngineArgs& A, const BlockCtx& B, const Team<BLOCK
             }
             int base_f = 0, base_b = 0;
             if (lane == 31) {
-                if (incl & 0xffff) base_f = atomicAdd(team.ctl + 2, incl & 0xffff);
-                if (incl >> 16) base_b = atomicAdd(team.ctl + 3, incl >> 16);
+                if (incl & 0xffff) base_f = atomicAdd(team.ctl + TC_OVERLAP, incl & 0xffff);
+                if (incl >> 16) base_b = atomicAdd(team.ctl + TC_OTHERS, incl >> 16);
             }
             base_f = __shfl_sync(0xffffffffu, base_f, 31);
             base_b = __shfl_sync(0xffffffffu, base_b, 31);
@@ -377,12 +450,12 @@ __device__ int icm_pair(const EngineArgs& A, const BlockCtx& B, const Team<BLOCK
             const int i = base + team.tr, i2 = i + team.ts;
             int8_t a = 0, b = 0, a2 = 0, b2 = 0;
             if (i < n) {
-                a = locA ? sA[i] : ld_cg(pubA + i);
-                b = locB ? sB[i] : ld_cg(pubB + i);
+                a = locA ? sA[i] : pub_site(pubA, i);
+                b = locB ? sB[i] : pub_site(pubB, i);
             }
             if (i2 < n) {
-                a2 = locA ? sA[i2] : ld_cg(pubA + i2);
-                b2 = locB ? sB[i2] : ld_cg(pubB + i2);
+                a2 = locA ? sA[i2] : pub_site(pubA, i2);
+                b2 = locB ? sB[i2] : pub_site(pubB, i2);
             }
             if (i < n) overlap_site(i, a, b);
             if (i2 < n) overlap_site(i2, a2, b2);
@@ -394,18 +467,55 @@ __device__ int icm_pair(const EngineArgs& A, const BlockCtx& B, const Team<BLOCK
     }
     if (algo == ENGINE_ICM_BFS)   // the visited bits of the breadth-first search
         for (int w = team.tr; w < nwords; w += team.ts) X.vis[w] = 0u;
-    team.reduce(cnt, kd, ke, hs);
-    const bool gflip = cnt > (long long)(n / 2);
+    // the overlap's size and whether any word was stale; every warp's best
+    // seed candidates (a block team takes the one it needs after the barrier)
+    bool again;
+    if (!REPLAY) {
+        kd = warp_min(kd);
+        ke = warp_min(ke);
+    }
+    if (BLOCK) {
+        if (!REPLAY && (threadIdx.x & 31) == 0) {
+            team.keys[2 * (threadIdx.x >> 5)] = kd;
+            team.keys[2 * (threadIdx.x >> 5) + 1] = ke;
+        }
+        if (stale) *(volatile int*)(team.ctl + TC_STALE) = 1;
+        __syncthreads();
+        cnt = *(volatile int*)(team.ctl + TC_OVERLAP);
+        again = *(volatile int*)(team.ctl + TC_STALE) != 0;
+    } else {
+        cnt = __reduce_add_sync(0xffffffffu, cnt);
+        again = __any_sync(0xffffffffu, stale);
+    }
+    if (!again) break;
+    // a partner's word had not arrived (its block published it before the
+    // energy this block waited for, but nothing orders the two): once more,
+    // at most as long as any wait on another block (a pass takes over 500 ns)
+    const unsigned long long limit = A.wait_limit_ns ? A.wait_limit_ns : kWaitLimitNs;
+    team.sync();
+    if (BLOCK && team.tr == 0) { team.ctl[TC_OVERLAP] = 0; team.ctl[TC_OTHERS] = 0; team.ctl[TC_STALE] = 0; }
+    team.sync();
+    if (tries > limit / 500) {
+        // (the run ends with this error at the group's next meeting)
+        if (team.tr == 0) dev_fail(A.status, A.abort_flag, DEV_BARRIER_TIMEOUT, 4, blockIdx.x, tag);
+        return 0;
+    }
+    stale = false;
+    cnt = 0;
+    kd = ke = ~0ull;
+    }
+    const bool gflip = cnt > n / 2;
     if (forced >= 0 && (d[forced] != 0) == gflip) {
         // a caller's seed must be a differing site after the global flip:
         // report it before any state changes (and clear the list counters)
         if (team.tr == 0) dev_fail(A.status, A.abort_flag, DEV_BAD_INDEX, where_err + 6, q, forced);
-        if (BLOCK && team.tr == 0) { team.ctl[2] = 0; team.ctl[3] = 0; team.ctl[4] = 0; }
+        team.sync();
+        if (BLOCK && team.tr == 0) { team.ctl[TC_OVERLAP] = 0; team.ctl[TC_OTHERS] = 0; team.ctl[TC_S] = 0; }
         team.sync();
         return 0;
     }
     // the overlap list of a block team: [l0, l0 + llen) of lst
-    const int l0 = gflip ? (int)cnt : 0, llen = gflip ? n - (int)cnt : (int)cnt;
+    const int l0 = gflip ? cnt : 0, llen = gflip ? n - cnt : cnt;
     auto for_overlap = [&](auto&& f) {
         if (BLOCK) {
             for (int t = team.tr; t < llen; t += team.ts) f(lst[l0 + t]);
@@ -417,14 +527,18 @@ __device__ int icm_pair(const EngineArgs& A, const BlockCtx& B, const Team<BLOCK
     long long dEa = 0, dEb = 0;
     if (gflip) {
         for (int i = team.tr; i < n; i += team.ts) {
-            if (locA) { sA[i] = (int8_t)-sA[i]; if (fA) fA[i] = -fA[i]; }
+            if (locA) {
+                const int a = sA[i];
+                if (has_h) dEa -= 2 * bh[i] * a;   // E(-s) = E(s) - 2 sum h s
+                sA[i] = (int8_t)-a;
+                if (fA) fA[i] = -fA[i];
+            }
             d[i] ^= 1;
         }
         cnt = n - cnt;
-        if (team.tr == 0) dEa = -2 * hs;   // E(-s) = E(s) - 2 sum h s
         team.sync();
     }
-    if (threadIdx.x == 0) P.subtick(PROF_ICM_DIFF);
+    P.subtick(PROF_ICM_DIFF);
     int seed = -1;
     if (REPLAY) {
         const long long idx = (long long)ls * D.nc + q;
@@ -445,13 +559,19 @@ __device__ int icm_pair(const EngineArgs& A, const BlockCtx& B, const Team<BLOCK
             }
         }
     } else if (cnt > 0) {
-        seed = forced >= 0 ? forced : (int)((gflip ? ke : kd) & 0xFFFFFFFFull);
+        if (BLOCK) {
+            const int lane = threadIdx.x & 31;
+            kd = warp_min(lane < (team.ts >> 5) ? team.keys[2 * lane + (gflip ? 1 : 0)] : ~0ull);
+        } else if (gflip) {
+            kd = ke;
+        }
+        seed = forced >= 0 ? forced : (int)(kd & 0xFFFFFFFFull);
         if (seed < 0 || seed >= n) {
             if (team.tr == 0) dev_fail(A.status, A.abort_flag, DEV_BAD_INDEX, where_err + 4, q, seed);
             return 0;
         }
     }
-    if (threadIdx.x == 0) P.subtick(PROF_ICM_SEED);
+    P.subtick(PROF_ICM_SEED);
     bool absolute = false;   // energies set from scratch (large flipped sets)
     int swapped = 0;         // the flipped set was D\C (the chains hold each other's result)
     // a block team's union-find lists the sites it found outside the giant
@@ -460,9 +580,9 @@ __device__ int icm_pair(const EngineArgs& A, const BlockCtx& B, const Team<BLOCK
     // (fast_eq) or is not (!fast_eq) fast_root
     bool fast = false, fast_eq = false;
     int fast_root = -1, ns = 0;
-    const int sbase = l0 == 0 ? llen : 0;
+    int sbase = l0 == 0 ? llen : 0;
     if (cnt > 0) {
-        long long csize = 0;
+        int csize = 0;
         if (algo == ENGINE_ICM_BFS) {
             // breadth-first search from the seed; members of C get d = 2
             // (the visited bits make each site's claim unique)
@@ -471,13 +591,13 @@ __device__ int icm_pair(const EngineArgs& A, const BlockCtx& B, const Team<BLOCK
                 X.queue[0] = seed;
                 X.vis[seed >> 5] |= 1u << (seed & 31);
                 d[seed] = 2;
-                vctl[1] = 1;
+                vctl[TC_TAIL] = 1;
             }
             team.sync();
             const int lane = threadIdx.x & 31;
             int lo = 0;
             for (int level = 0; level <= n; level++) {
-                const int hi = vctl[1];
+                const int hi = vctl[TC_TAIL];
                 team.sync();
                 if (lo == hi) break;
                 for (int base = lo; base < hi; base += team.ts) {
@@ -500,7 +620,7 @@ __device__ int icm_pair(const EngineArgs& A, const BlockCtx& B, const Team<BLOCK
                         if (m) {
                             const int leader = __ffs(m) - 1;
                             int slot0 = 0;
-                            if (lane == leader) slot0 = atomicAdd(team.ctl + 1, __popc(m));
+                            if (lane == leader) slot0 = atomicAdd(team.ctl + TC_TAIL, __popc(m));
                             slot0 = __shfl_sync(0xffffffffu, slot0, leader);
                             if (found) {
                                 X.queue[slot0 + __popc(m & ((1u << lane) - 1u))] = v;
@@ -513,7 +633,7 @@ __device__ int icm_pair(const EngineArgs& A, const BlockCtx& B, const Team<BLOCK
                 lo = hi;
             }
             csize = lo;
-            if (threadIdx.x == 0) P.subtick(PROF_ICM_UNION);
+            P.subtick(PROF_ICM_UNION);
         } else {
             // label the components of the whole overlap subgraph, then mark the
             // sites sharing the seed's label
@@ -525,24 +645,111 @@ __device__ int icm_pair(const EngineArgs& A, const BlockCtx& B, const Team<BLOCK
                 for (int i = team.tr; i < n; i += team.ts) lab[i] = d[i] ? i : n;
                 team.sync();
             }
-            if (algo == ENGINE_ICM_UNION_FIND) {
+            // (few neighbours: every edge is a link, nothing to sample)
+            const bool direct = algo == ENGINE_ICM_UNION_FIND && D.nnz <= kDirectDegree * n && n <= kDirectSites && D.ncolors <= 3;
+            if (direct) {
+                // every edge from its upper end: each site is hooked under
+                // its lowest overlap neighbour below it by a plain store,
+                // then united with the others below it
+                for_overlap([&](int u) {
+                    int lo = u;
+                    const int e1 = brow[u + 1];
+#pragma unroll 4
+                    for (int a = brow[u]; a < e1; a++) {
+                        const int v = (int)(badj[a] >> 8);
+                        if (v < lo && d[v]) lo = v;
+                    }
+                    if (lo < u) lab[u] = lo;
+                });
+                team.sync();
+                P.subtick(PROF_UF_LINK0);
+                for_overlap([&](int u) {
+                    const int e1 = brow[u + 1];
+                    int lo = u;
+#pragma unroll 4
+                    for (int a = brow[u]; a < e1; a++) {
+                        const int v = (int)(badj[a] >> 8);
+                        if (v < lo && d[v]) lo = v;
+                    }
+                    for (int a = brow[u]; a < e1; a++) {
+                        const int v = (int)(badj[a] >> 8);
+                        if (v < u && v != lo && d[v]) ok &= uf_unite(lab, u, v);
+                    }
+                });
+                team.sync();
+                P.subtick(PROF_UF_LINK1);
+                if (BLOCK) {
+                    // the cluster's size, and the flipped set from the list
+                    const int rs = uf_find(vl, seed);
+                    int c = 0;
+                    for (int t = team.tr; t < llen; t += team.ts) c += uf_find(vl, lst[l0 + t]) == rs;
+                    csize = team.count(c);
+                    if (team.tr == 0) { team.ctl[TC_OVERLAP] = 0; team.ctl[TC_OTHERS] = 0; }
+                    fast = true;
+                    fast_root = rs;
+                    fast_eq = exact || csize * 2 <= cnt;
+                    sbase = l0;
+                    ns = llen;
+                    P.subtick(PROF_UF_SIZE);
+                }
+            } else if (algo == ENGINE_ICM_UNION_FIND) {
                 // Afforest (Sutton, Ben-Nun, Barak, IPDPS 2018): in two
-                // rounds, link every overlap site to its r-th overlap
-                // neighbour and compress the trees; take the most frequent
+                // rounds, link every overlap site to its first two overlap
+                // neighbours and compress the trees in between; take the most frequent
                 // root of a sample as the large component L, then process the
                 // full adjacency only of sites outside L.  An edge skipped at
                 // an end in L is processed from its other end, unless that end
                 // is in L too -- then both are already joined.
                 // (GLINK: with the neighbour lists in device memory, a
                 // thread scans four of its sites side by side, so that
-                // their dependent loads overlap, then makes their unions)
-                const bool glink = GLINK && BLOCK && !__isShared(badj);
-                // (a block team's round 0 also finds each site's second
-                // overlap neighbour and keeps it, by list position, in the
-                // free part of the list -- S is listed there only later --
-                // for round 1)
+                // their dependent loads overlap)
+                const bool glink = GLINK && BLOCK && (SPACE == SP_LARGE || !__isShared(badj)) &&
+                                   (reinterpret_cast<uintptr_t>(badj) & 15u) == 0;
+                // (a block team's round 0 keeps the link left for round 1, by
+                // list position, in the free part of the list: S is listed
+                // there only later)
                 int* const link1 = (BLOCK && (LS || GLINK)) ? lst + sbase : nullptr;
-                for (int round = 0; round < 2; round++) {
+                // u's first two overlap neighbours (-1: none): the list four
+                // entries at a time, four independent loads, then four flags
+                auto first_two = [&](int u, int& v0, int& v1) {
+                    v0 = v1 = -1;
+                    const int e1 = brow[u + 1];
+                    for (int a = brow[u]; a < e1 && v1 < 0; a += 4) {
+                        int v[4];
+                        bool on[4];
+#pragma unroll
+                        for (int j = 0; j < 4; j++) v[j] = a + j < e1 ? (int)(badj[a + j] >> 8) : u;
+#pragma unroll
+                        for (int j = 0; j < 4; j++) on[j] = a + j < e1 && d[v[j]];
+#pragma unroll
+                        for (int j = 0; j < 4; j++)
+                            if (on[j]) {
+                                if (v0 < 0) v0 = v[j];
+                                else if (v1 < 0) v1 = v[j];
+                            }
+                    }
+                };
+                // Round 0 hooks u under the lower of the two when that lies
+                // below u: a plain store by u's own thread, no find and no
+                // compare-and-swap (parents strictly decrease, so no cycle;
+                // unions by find walked trees that nothing had compressed
+                // yet).  Round 1 unites u with what the hook left, after the
+                // compression.  (In round 1 of a team without kept targets
+                // the hook's outcome is found again and not stored.)
+                int round = 0;
+                auto hook = [&](int u, int v0, int v1) {
+                    const int lo = v1 >= 0 && v1 < v0 ? v1 : v0;
+                    if (lo < 0) return -1;
+                    if (lo > u) {
+                        // (not hooked: the second neighbour may hang under u;
+                        // whichever of two parents is stored, it is a link)
+                        if (round == 0 && v1 >= 0) atomicMin(lab + v1, u);
+                        return v0;
+                    }
+                    if (round == 0) lab[u] = lo;
+                    return v1 < 0 ? -1 : (lo == v0 ? v1 : v0);
+                };
+                for (round = 0; round < 2; round++) {
                     if (round == 1 && link1 != nullptr) {
                         for (int t = team.tr; t < llen; t += 4 * team.ts) {
                             int u[4], tg[4];
@@ -557,8 +764,15 @@ __device__ int icm_pair(const EngineArgs& A, const BlockCtx& B, const Team<BLOCK
                                 if (u[k] >= 0 && tg[k] >= 0) ok &= uf_unite(lab, u[k], tg[k]);
                         }
                     } else if (glink) {
+                        // four list sites at a time, each with the two 16-byte
+                        // pieces of its list that hold its first entries (five
+                        // to eight of them: usually both targets).  The loads
+                        // are scattered, so what they cost is one L1 lookup
+                        // per lane and load: two pieces instead of eight
+                        // entries
+                        const uint4* const adj4 = reinterpret_cast<const uint4*>(badj);
                         for (int t = team.tr; t < llen; t += 4 * team.ts) {
-                            int u[4], a[4], e[4], tg[4], k4[4];
+                            int u[4], a[4], e[4];
 #pragma unroll
                             for (int k = 0; k < 4; k++) {
                                 const int tk = t + k * team.ts;
@@ -569,99 +783,64 @@ __device__ int icm_pair(const EngineArgs& A, const BlockCtx& B, const Team<BLOCK
                                 a[k] = u[k] >= 0 ? brow[u[k]] : 0;
                                 e[k] = u[k] >= 0 ? brow[u[k] + 1] : 0;
                             }
-                            uint32_t v[4][4];
+                            int v0[4], v1[4];
 #pragma unroll
-                            for (int k = 0; k < 4; k++)
+                            for (int k = 0; k < 4; k++) v0[k] = v1[k] = -1;
+                            // 16-byte pieces j and j + 1 of the sites whose
+                            // links are not both found, all loads before their
+                            // use
+                            for (int j0 = 0;; j0 += 2) {
+                                uint4 p[4][2];
+                                bool more = false;
 #pragma unroll
-                                for (int j = 0; j < 4; j++) v[k][j] = a[k] + j < e[k] ? badj[a[k] + j] : 0xFFFFFFFFu;
-                            // the round-th overlap neighbour (tg) and, in
-                            // round 0 with a place to keep it, the next (t1)
-                            const int want = (round == 0 && link1 != nullptr) ? 2 : round + 1;
-                            int t1[4];
+                                for (int k = 0; k < 4; k++)
 #pragma unroll
-                            for (int k = 0; k < 4; k++) {
-                                tg[k] = -1;
-                                t1[k] = -1;
-                                k4[k] = 0;
+                                    for (int j = 0; j < 2; j++)
+                                        p[k][j] = v1[k] < 0 && 4 * ((a[k] >> 2) + j0 + j) < e[k] ? adj4[(a[k] >> 2) + j0 + j]
+                                                                                                 : make_uint4(0, 0, 0, 0);
 #pragma unroll
-                                for (int j = 0; j < 4; j++) {
-                                    const bool on = v[k][j] != 0xFFFFFFFFu && d[v[k][j] >> 8];
-                                    if (on && k4[k] < want) {
-                                        if (k4[k] == round) tg[k] = (int)(v[k][j] >> 8);
-                                        else if (k4[k] == round + 1) t1[k] = (int)(v[k][j] >> 8);
-                                        k4[k]++;
+                                for (int k = 0; k < 4; k++) {
+                                    const int b0 = (a[k] & ~3) + 4 * j0;
+                                    const uint32_t w8[8] = {p[k][0].x, p[k][0].y, p[k][0].z, p[k][0].w,
+                                                            p[k][1].x, p[k][1].y, p[k][1].z, p[k][1].w};
+#pragma unroll
+                                    for (int x = 0; x < 8; x++) {
+                                        const int v = (int)(w8[x] >> 8);
+                                        if (v1[k] < 0 && b0 + x >= a[k] && b0 + x < e[k] && d[v]) {
+                                            if (v0[k] < 0) v0[k] = v;
+                                            else v1[k] = v;
+                                        }
                                     }
+                                    more |= v1[k] < 0 && b0 + 8 < e[k];
                                 }
+                                if (!more) break;
                             }
 #pragma unroll
                             for (int k = 0; k < 4; k++) {
                                 if (u[k] < 0) continue;
-                                // the targets past the first four entries: four
-                                // independent loads at a time
-                                for (int aa = a[k] + 4; aa < e[k] && k4[k] < want; aa += 4) {
-                                    uint32_t w4[4];
-#pragma unroll
-                                    for (int j = 0; j < 4; j++) w4[j] = aa + j < e[k] ? badj[aa + j] : 0xFFFFFFFFu;
-#pragma unroll
-                                    for (int j = 0; j < 4; j++) {
-                                        const bool on = w4[j] != 0xFFFFFFFFu && d[w4[j] >> 8];
-                                        if (on && k4[k] < want) {
-                                            if (k4[k] == round) tg[k] = (int)(w4[j] >> 8);
-                                            else if (k4[k] == round + 1) t1[k] = (int)(w4[j] >> 8);
-                                            k4[k]++;
-                                        }
-                                    }
-                                }
-                                if (round == 0 && link1 != nullptr) link1[t + k * team.ts] = t1[k];
-                                if (tg[k] >= 0) ok &= uf_unite(lab, u[k], tg[k]);
+                                const int rest = hook(u[k], v0[k], v1[k]);
+                                if (link1 != nullptr) link1[t + k * team.ts] = rest;
+                                else if (round == 1 && rest >= 0) ok &= uf_unite(lab, u[k], rest);
                             }
                         }
                     } else if (link1 != nullptr) {
-                        // round 0 of a block team: the first two overlap
-                        // neighbours, the list four entries at a time
+                        // round 0 of a block team: the list four entries at a
+                        // time
                         for (int t = team.tr; t < llen; t += team.ts) {
                             const int u = lst[l0 + t];
-                            int k = 0, tgt = -1, t1 = -1;
-                            const int e1 = brow[u + 1];
-                            for (int a = brow[u]; a < e1 && k < 2; a += 4) {
-                                int v[4];
-                                bool on[4];
-#pragma unroll
-                                for (int j = 0; j < 4; j++) v[j] = a + j < e1 ? (int)(badj[a + j] >> 8) : u;
-#pragma unroll
-                                for (int j = 0; j < 4; j++) on[j] = a + j < e1 && d[v[j]];
-#pragma unroll
-                                for (int j = 0; j < 4; j++)
-                                    if (on[j] && k < 2) {
-                                        if (k == 0) tgt = v[j];
-                                        else t1 = v[j];
-                                        k++;
-                                    }
-                            }
-                            link1[t] = t1;
-                            if (tgt >= 0) ok &= uf_unite(lab, u, tgt);
+                            int v0, v1;
+                            first_two(u, v0, v1);
+                            link1[t] = hook(u, v0, v1);
                         }
                     } else
                     for_overlap([&](int u) {
-                        // the neighbour list four entries at a time: four
-                        // independent loads, then four flag loads
-                        int k = 0, tgt = -1;
-                        const int e1 = brow[u + 1];
-                        for (int a = brow[u]; a < e1 && tgt < 0; a += 4) {
-                            int v[4];
-                            bool on[4];
-#pragma unroll
-                            for (int j = 0; j < 4; j++) v[j] = a + j < e1 ? (int)(badj[a + j] >> 8) : u;
-#pragma unroll
-                            for (int j = 0; j < 4; j++) on[j] = a + j < e1 && d[v[j]];
-#pragma unroll
-                            for (int j = 0; j < 4; j++)
-                                if (on[j] && tgt < 0 && k++ == round) tgt = v[j];
-                        }
-                        if (tgt >= 0) ok &= uf_unite(lab, u, tgt);
+                        int v0, v1;
+                        first_two(u, v0, v1);
+                        const int rest = hook(u, v0, v1);
+                        if (round == 1 && rest >= 0) ok &= uf_unite(lab, u, rest);
                     });
                     team.sync();
-                    if (threadIdx.x == 0) P.subtick(round == 0 ? PROF_UF_LINK0 : PROF_UF_LINK1);
+                    P.subtick(round == 0 ? PROF_UF_LINK0 : PROF_UF_LINK1);
                     if (round == 0) {
                         // (after the last round the vote's and phase 3's
                         // finds halve the paths they walk)
@@ -689,7 +868,7 @@ __device__ int icm_pair(const EngineArgs& A, const BlockCtx& B, const Team<BLOCK
                             else vl[u] = r;
                         });
                         team.sync();
-                        if (threadIdx.x == 0) P.subtick(PROF_UF_COMPRESS);
+                        P.subtick(PROF_UF_COMPRESS);
                     }
                 }
                 int L = -1;
@@ -725,18 +904,18 @@ __device__ int icm_pair(const EngineArgs& A, const BlockCtx& B, const Team<BLOCK
                         if (ov > votes || (ov == votes && oc < best)) { votes = ov; best = oc; }
                     }
                     if (BLOCK) L = best;
-                    else if (team.tr == 0) team.ctl[0] = best;
+                    else if (team.tr == 0) team.ctl[TC_BEST] = best;
                 }
                 if (!BLOCK) {
                     team.sync();
                     L = *(volatile int*)team.ctl;
                 }
-                if (threadIdx.x == 0) P.subtick(PROF_UF_VOTE);
+                P.subtick(PROF_UF_VOTE);
                 for_overlap([&](int u) {
                     if (uf_find(vl, u) == L) return;
                     if (BLOCK) {
                         // S never outgrows the free part of lst: |S| <= llen <= n - llen
-                        const int pos = atomicAdd(team.ctl + 4, 1);
+                        const int pos = atomicAdd(team.ctl + TC_S, 1);
                         if (pos < llen) lst[sbase + pos] = u;
                         return;
                     }
@@ -748,12 +927,12 @@ __device__ int icm_pair(const EngineArgs& A, const BlockCtx& B, const Team<BLOCK
                     }
                 });
                 team.sync();
-                if (threadIdx.x == 0) P.subtick(PROF_UF_OUTSIDE);
+                P.subtick(PROF_UF_OUTSIDE);
                 if (BLOCK) {
                     // the edges of S: one warp per site and one lane per
                     // neighbour (the unions of a site side by side) when
                     // that takes fewer rounds than one thread per site
-                    const int ns0 = min(*(volatile int*)(team.ctl + 4), llen);
+                    const int ns0 = min(*(volatile int*)(team.ctl + TC_S), llen);
                     const int nw = team.ts >> 5;
                     const bool by_warp = (ns0 + nw - 1) / nw < (D.nnz + n - 1) / n;
                     const int t0 = by_warp ? team.tr >> 5 : team.tr, dt = by_warp ? nw : team.ts;
@@ -767,31 +946,29 @@ __device__ int icm_pair(const EngineArgs& A, const BlockCtx& B, const Team<BLOCK
                         }
                     }
                     team.sync();
-                    if (threadIdx.x == 0) P.subtick(PROF_UF_SUNION);
+                    P.subtick(PROF_UF_SUNION);
                 }
                 if (BLOCK) {
                     // sites in L's component at their phase-3 check stay in it:
                     // every site outside the final component of L is in S
-                    ns = min(*(volatile int*)(team.ctl + 4), llen);
+                    ns = min(*(volatile int*)(team.ctl + TC_S), llen);
                     const int rL = uf_find(vl, L), rs = uf_find(vl, seed);
-                    long long c = 0;   // |S \ comp(L)| when the seed is in comp(L), else |C|
+                    int c = 0;   // |S \ comp(L)| when the seed is in comp(L), else |C|
                     for (int t = team.tr; t < ns; t += team.ts) {
                         const int r = uf_find(vl, lst[sbase + t]);
                         c += (rs == rL) ? (r != rL) : (r == rs);
                     }
-                    unsigned long long m1 = ~0ull, m2 = ~0ull;
-                    long long none = 0;
-                    team.reduce(c, m1, m2, none);
+                    c = team.count(c);
                     // every thread has read the list counters: reset them
                     // for the next pair (a barrier of this pair's flip or
                     // energy reduction comes before its next use)
-                    if (team.tr == 0) { team.ctl[2] = 0; team.ctl[3] = 0; team.ctl[4] = 0; }
+                    if (team.tr == 0) { team.ctl[TC_OVERLAP] = 0; team.ctl[TC_OTHERS] = 0; team.ctl[TC_S] = 0; }
                     csize = (rs == rL) ? cnt - c : c;
                     const bool sw = !exact && csize * 2 > cnt;
                     fast = (rs == rL) ? sw : !sw;   // the flipped set lies in S
                     fast_root = rs == rL ? rL : rs;
                     fast_eq = rs != rL;
-                    if (threadIdx.x == 0) P.subtick(PROF_UF_SIZE);
+                    P.subtick(PROF_UF_SIZE);
                 }
             } else {
                 // minimum-label propagation with root hooking and pointer jumping
@@ -834,7 +1011,7 @@ __device__ int icm_pair(const EngineArgs& A, const BlockCtx& B, const Team<BLOCK
                 ok = conv;
             }
             if (!ok) dev_fail(A.status, A.abort_flag, DEV_UF_LIMIT, where_err + 3, q, algo);
-            if (threadIdx.x == 0) P.subtick(PROF_ICM_UNION);
+            P.subtick(PROF_ICM_UNION);
             const int root = (algo == ENGINE_ICM_UNION_FIND) ? uf_find(vl, seed) : vl[seed];
             if (BLOCK && algo == ENGINE_ICM_UNION_FIND) {
                 // csize is known.  When the flipped set is not in S it is the
@@ -855,9 +1032,7 @@ __device__ int icm_pair(const EngineArgs& A, const BlockCtx& B, const Team<BLOCK
                     d[u] = 2;
                     csize++;
                 });
-                unsigned long long m1 = ~0ull, m2 = ~0ull;
-                long long none = 0;
-                team.reduce(csize, m1, m2, none);
+                csize = team.count(csize);
             }
         }
         // (A, B) -> (A flipped on C, B flipped on C) is the same pair of
@@ -869,7 +1044,7 @@ __device__ int icm_pair(const EngineArgs& A, const BlockCtx& B, const Team<BLOCK
         // invariant.  Replay keeps the reference's flips.
         swapped = (!exact && csize * 2 > cnt) ? 1 : 0;
         const uint8_t fmark = swapped ? 1 : 2;
-        const long long fsize = swapped ? cnt - csize : csize;
+        const int fsize = swapped ? cnt - csize : csize;
         // membership of an overlap site in the flipped set
         const bool rest = BLOCK && algo == ENGINE_ICM_UNION_FIND && !fast;
         auto in_flip = [&](int u) { return rest ? d[u] != 3 : d[u] == fmark; };
@@ -915,7 +1090,7 @@ __device__ int icm_pair(const EngineArgs& A, const BlockCtx& B, const Team<BLOCK
                 const int u = lst[sbase + t];
                 if ((uf_find((volatile int*)X.queue, u) == fast_root) == fast_eq) flip_push(u, by_warp);
             }
-        } else if (BLOCK && fsize * 4 > (long long)n) {
+        } else if (BLOCK && (long long)fsize * 4 > (long long)n) {
             // a large cluster: flip, then fields and energies from scratch
             // (gathers, no atomics; the cost does not grow with the cluster)
             for_overlap([&](int u) {
@@ -940,7 +1115,7 @@ __device__ int icm_pair(const EngineArgs& A, const BlockCtx& B, const Team<BLOCK
                 if (locA) { if (fA) fA[i] = fa; eA += (long long)sA[i] * (h2 + fa); }
                 if (locB) { if (fB) fB[i] = fb; eB += (long long)sB[i] * (h2 + fb); }
             }
-            team.sum2(eA, eB);
+            team.sum_energies(eA, eB, A.small_energy != 0);
             if (team.tr == 0) {
                 if (locA) B.E[rA] = eA / 2;
                 if (locB) B.E[rB] = eB / 2;
@@ -952,10 +1127,10 @@ __device__ int icm_pair(const EngineArgs& A, const BlockCtx& B, const Team<BLOCK
                 if (in_flip(u)) flip_push(u, false);
             });
         }
-        team.sync();
+        if (!BLOCK || absolute) team.sync();   // (a block team's energy sums have the barrier)
     }
     if (!absolute && (gflip || cnt > 0)) {
-        team.sum2(dEa, dEb);
+        team.sum_energies(dEa, dEb, A.small_energy != 0);
         if (team.tr == 0) {
             if (locA) B.E[rA] += dEa;
             if (locB && cnt > 0) B.E[rB] += dEb;
@@ -965,16 +1140,14 @@ __device__ int icm_pair(const EngineArgs& A, const BlockCtx& B, const Team<BLOCK
         // (a block team's union-find reset the list counters after its size
         // reduction and passed a barrier since)
         if (BLOCK && team.tr == 0) {
-            team.ctl[2] = 0;   // the list counters, for the next pair
-            team.ctl[3] = 0;
-            team.ctl[4] = 0;
+            team.ctl[TC_OVERLAP] = 0;   // the list counters, for the next pair
+            team.ctl[TC_OTHERS] = 0;
+            team.ctl[TC_S] = 0;
         }
         team.sync();
     }
-    if (threadIdx.x == 0) {
-        P.subtick(PROF_ICM_FLIP);
-        if (P.on && cnt > 0) P.c[PROF_ICM_COUNT]++;
-    }
+    P.subtick(PROF_ICM_FLIP);
+    if (P.on && cnt > 0) P.s->c[PROF_ICM_COUNT]++;
     return swapped;
 }
 
@@ -1022,12 +1195,9 @@ __device__ void colored_sweep(const EngineArgs& A, const BlockCtx& B, unsigned l
     unsigned acc_fl = 0;
     // several replicas in the block, fields gathered
     const bool gm = !ONE && B.field == nullptr && rpc <= kGatherReps;
-    // the one-replica sweep's pointers and flags, read once from the
-    // block's shared context (the compiler may not keep them across the
-    // stores of a colour class)
     int8_t* const sp1 = B.spin;
     int32_t* const fd1 = B.field;
-    const int32_t* const h1 = D.has_h ? B.h : nullptr;
+    const int32_t* const h1 = B.h;
     const uint32_t* const thr1 = ONE ? s_thr + B.tb[0] : s_thr;
     const int ncolors = D.ncolors;
     for (int c = 0; c < ncolors; c++) {
@@ -1090,7 +1260,7 @@ __device__ void colored_sweep(const EngineArgs& A, const BlockCtx& B, unsigned l
             const uint32_t* thr_row = s_thr + B.tb[0];
             for (int i = c0 + tid; i < c0 + Sc; i += T) {
                 const int s = sp[i];
-                const int f = (fd ? fd[i] : gather_field(row, adj, sp, i)) + (D.has_h ? B.h[i] : 0);
+                const int f = (fd ? fd[i] : gather_field(row, adj, sp, i)) + (B.h ? B.h[i] : 0);
                 const int de = -2 * s * f;
                 bool acc = de <= 0;
                 if (!acc) {
@@ -1148,7 +1318,7 @@ __device__ void colored_sweep(const EngineArgs& A, const BlockCtx& B, unsigned l
                     for (int j = 0; j < kGatherReps; j++)
                         if (j < rpc) f[j] += w * sn[j * npad];
                 });
-                const int hi = D.has_h ? B.h[i] : 0;
+                const int hi = B.h ? B.h[i] : 0;
 #pragma unroll
                 for (int j = 0; j < kGatherReps; j++) {
                     if (j < rpc) {
@@ -1195,7 +1365,7 @@ __device__ void colored_sweep(const EngineArgs& A, const BlockCtx& B, unsigned l
                     int8_t* sp = B.spin + j * npad;
                     int32_t* fd = B.field ? B.field + j * npad : nullptr;
                     const int s = sp[i];
-                    const int f = (fd ? fd[i] : gather_field(row, adj, sp, i)) + (D.has_h ? B.h[i] : 0);
+                    const int f = (fd ? fd[i] : gather_field(row, adj, sp, i)) + (B.h ? B.h[i] : 0);
                     de = -2 * s * f;
                     acc = de <= 0;
                     if (!acc) {
@@ -1297,7 +1467,7 @@ __device__ void replay_sweep(const EngineArgs& A, const BlockCtx& B, int ls, int
             int acc = 0, s = 0, de = 0;
             if (lane == 0) {
                 s = sp[i];
-                const int f = fd[i] + (D.has_h ? B.h[i] : 0);
+                const int f = fd[i] + (B.h ? B.h[i] : 0);
                 de = -2 * s * f;
                 if (de <= 0) {
                     acc = 1;
@@ -1352,8 +1522,8 @@ __device__ void replay_sweep(const EngineArgs& A, const BlockCtx& B, int ls, int
 __device__ void exchange_reference_order(const EngineArgs& A, const BlockCtx& B, unsigned long long step,
                                          uint32_t* s_order, const double* s_dbeta, unsigned* s_att,
                                          unsigned* s_succ, float* s_xlogu, uint32_t* s_xrand,
-                                         int* s_lvl, uint32_t* s_tmp, int* s_misc, Prof& P) {
-    if (threadIdx.x == 0) P.subtick(PROF_X_SHUFFLE);
+                                         int* s_lvl, uint32_t* s_tmp, int* s_misc, const Prof P) {
+    P.subtick(PROF_X_SHUFFLE);
     const InstanceDesc& D = B.D;
     const int tid = threadIdx.x, T = blockDim.x;
     const int nt = D.nt, C = D.chains, m = nt - 1;
@@ -1374,7 +1544,7 @@ __device__ void exchange_reference_order(const EngineArgs& A, const BlockCtx& B,
         }
     }
     __syncthreads();
-    if (threadIdx.x == 0) P.subtick(PROF_X_DRAW);
+    P.subtick(PROF_X_DRAW);
     // one warp walks the rounds; the rest of the block waits at the end
     if (tid < 32) {
         const int lane = tid;
@@ -1409,7 +1579,7 @@ __device__ void exchange_reference_order(const EngineArgs& A, const BlockCtx& B,
             int maxl = 0;
             for (int i = lane; i < m; i += 32) maxl = max(maxl, s_lvl[i]);
             const int L = __reduce_max_sync(0xffffffffu, maxl);
-            if (lane == 0) P.subtick(PROF_X_LEVELS);
+            P.subtick(PROF_X_LEVELS);
             for (int lv = 1; lv <= L; lv++) {
                 for (int i = lane; i < m; i += 32) {
                     if (s_lvl[i] != lv) continue;
@@ -1428,7 +1598,7 @@ __device__ void exchange_reference_order(const EngineArgs& A, const BlockCtx& B,
                 }
                 __syncwarp();
             }
-            if (lane == 0) P.subtick(PROF_X_APPLY);
+            P.subtick(PROF_X_APPLY);
             // reshuffle: rank the pairs by fresh random keys (ties by position)
             const uint32_t* keys = s_xrand + round * m;
             for (int i = lane; i < m; i += 32) {
@@ -1443,54 +1613,82 @@ __device__ void exchange_reference_order(const EngineArgs& A, const BlockCtx& B,
             __syncwarp();
             for (int i = lane; i < m; i += 32) s_order[i] = s_tmp[i];
             __syncwarp();
-            if (lane == 0) P.subtick(PROF_X_SHUFFLE);
+            P.subtick(PROF_X_SHUFFLE);
         }
     }
     __syncthreads();
     (void)s_misc;
 }
 
+// Log-uniforms of the even/odd exchange: a thread's pair of each pass, drawn
+// before the step's energies are known (they do not depend on them).
+struct EvenOddDraws {
+    float lu0, lu1;
+};
+
+__device__ __forceinline__ float even_odd_log_u(unsigned long long seed, uint32_t inst, unsigned long long step, int k,
+                                                int par) {
+    const uint4 r = philox4x32_10(make_uint4((uint32_t)(k | (par << 30)), inst, (uint32_t)step, (uint32_t)(step >> 32)),
+                                  stream_key(seed, STREAM_EXCHANGE));
+    return __logf(u01_open0(r.x));
+}
+
+// The t-th pair of a pass (pairs kb = par, par + 2, ... of every chain).
+__device__ __forceinline__ int even_odd_pair(int t, int par, int per_chain, int nt, int& kb) {
+    const int c = t / per_chain;
+    kb = par + 2 * (t - c * per_chain);
+    return c * nt + kb;
+}
+
+__device__ __forceinline__ EvenOddDraws even_odd_draw(const EngineArgs& A, const InstanceDesc& D, unsigned long long step) {
+    const int nt = D.nt, C = D.chains, m = nt - 1, per0 = (m + 1) / 2, per1 = m / 2;
+    const int tid = threadIdx.x;
+    EvenOddDraws u{0.f, 0.f};
+    if (C * per0 > (int)blockDim.x) return u;   // (then drawn as the pairs are visited)
+    int kb;
+    if (tid < C * per0) u.lu0 = even_odd_log_u(A.seed, (uint32_t)D.inst_id, step, even_odd_pair(tid, 0, per0, nt, kb), 0);
+    if (tid < C * per1) u.lu1 = even_odd_log_u(A.seed, (uint32_t)D.inst_id, step, even_odd_pair(tid, 1, per1, nt, kb), 1);
+    return u;
+}
+
+// Accepts a swap with energy difference dE across dbeta: x = dbeta * dE > 0
+// or log u < x, in FP64.  The sign of x is the product of the signs, and the
+// comparison is decided in FP32 unless log u lies within 1e-5 of x relative
+// to |x| (the FP32 product is within 2^-21 of x), so that the FP64 pipe,
+// slow on this chip, is left to about one attempt in 10^5.
+__device__ __forceinline__ bool swap_accepted(double dbeta, long long dE, float log_u) {
+    const float db = (float)dbeta, xf = db * (float)dE;
+    if (dE == 0 && fabsf(db) < 1e30f) return log_u < 0.f;
+    if (fabsf(xf) > 1e-30f && fabsf(db) > 1e-30f) {
+        if (xf > 0.f) return true;
+        if (fabsf(log_u - xf) > 1e-5f * fabsf(xf)) return log_u < xf;
+    }
+    const double x = dbeta * (double)dE;
+    return x > 0.0 || (double)log_u < x;
+}
+
 // Deterministic even/odd exchange: per chain, all even pairs, then all odd
 // pairs, each set in parallel (nt-1 attempts per chain per step).
 __device__ void exchange_even_odd(const EngineArgs& A, const BlockCtx& B, unsigned long long step,
-                                  const double* s_dbeta, unsigned* s_att, unsigned* s_succ) {
+                                  const double* s_dbeta, unsigned* s_att, unsigned* s_succ, EvenOddDraws u) {
     const InstanceDesc& D = B.D;
     const int tid = threadIdx.x, T = blockDim.x;
     const int nt = D.nt, C = D.chains, m = nt - 1;
     const uint32_t inst = (uint32_t)D.inst_id;
     uint32_t* const slot = B.slot;
     const long long* const E = B.E;
-    const uint2 key = stream_key(A.seed, STREAM_EXCHANGE);
-    auto log_u = [&](int k, int par) {
-        const uint4 r = philox4x32_10(make_uint4((uint32_t)(k | (par << 30)), inst, (uint32_t)step, (uint32_t)(step >> 32)), key);
-        return __logf(u01_open0(r.x));
-    };
-    auto pair_of = [&](int t, int par, int per_chain, int& kb) {
-        const int c = t / per_chain;
-        kb = par + 2 * (t - c * per_chain);
-        return c * nt + kb;
-    };
-    // when each pass has at most one pair per thread, both passes' draws
-    // are made first, side by side (they do not depend on the energies)
     const int per0 = (m + 1) / 2, per1 = m / 2;
-    const bool one = C * per0 <= T;
-    float lu0 = 0.f, lu1 = 0.f;
-    if (one) {
-        int kb;
-        if (tid < C * per0) lu0 = log_u(pair_of(tid, 0, per0, kb), 0);
-        if (tid < C * per1) lu1 = log_u(pair_of(tid, 1, per1, kb), 1);
-    }
+    const bool one = C * per0 <= T;   // at most one pair per thread and pass: drawn ahead
     for (int par = 0; par < 2; par++) {
-        const int per_chain = par ? per1 : per0;   // pairs kb = par, par+2, ...
+        const int per_chain = par ? per1 : per0;
         const int total = C * per_chain;
         for (int t = tid; t < total; t += T) {
             int kb;
-            const int k = pair_of(t, par, per_chain, kb);
-            const float lu = one ? (par ? lu1 : lu0) : log_u(k, par);
+            const int k = even_odd_pair(t, par, per_chain, nt, kb);
+            const float lu = one ? (par ? u.lu1 : u.lu0) : even_odd_log_u(A.seed, inst, step, k, par);
             const uint32_t r1 = slot[k], r2 = slot[k + 1];
-            const double x = s_dbeta[kb] * (double)(E[r1] - E[r2]);
             s_att[k]++;
-            if (x > 0.0 || (double)lu < x) {
+            if (swap_accepted(s_dbeta[kb], E[r1] - E[r2], lu)) {
                 s_succ[k]++;
                 slot[k] = r2;
                 slot[k + 1] = r1;
@@ -1539,14 +1737,15 @@ __device__ void exchange_replay(const EngineArgs& A, const BlockCtx& B, int ls, 
 // run at most kNarrowThreads threads, which leaves each thread 120 registers
 // instead of the 64 of a 1024-thread bound; replay and wide block teams (one
 // replica of a large instance per block) keep 1024.
-template <bool REPLAY, bool BLOCKTEAM, bool NARROW>
+template <bool REPLAY, bool BLOCKTEAM, bool NARROW, int SPACE>
 __global__ void __launch_bounds__((REPLAY || (BLOCKTEAM && !NARROW)) ? 1024 : kNarrowThreads, 1)
     pt_engine_kernel(const EngineArgs A) {
     extern __shared__ __align__(128) uint8_t smem[];
-    // the job's context and the profiling counters: one copy per block (per-
-    // thread copies of uniform values would live in local memory)
-    __shared__ BlockCtx s_B;
-    __shared__ long long s_prof[PROF_PHASES];
+    // the job's descriptor and the profiling counters: one copy per block
+    // (per-thread copies of uniform values would live in local memory)
+    __shared__ InstanceDesc s_D;
+    __shared__ int s_rank;
+    __shared__ ProfStore s_prof;
     const SmemPlan& S = A.sm;
     const int tid = threadIdx.x, T = blockDim.x;
     volatile int* abortf = A.abort_flag;
@@ -1560,20 +1759,20 @@ __global__ void __launch_bounds__((REPLAY || (BLOCKTEAM && !NARROW)) ? 1024 : kN
     for (int job = A.sched_off[blockIdx.x]; job < job_end; job++) {
     const int inst = A.sched[2 * job];
     if (tid == 0) {
-        s_B.D = A.desc[inst];
-        s_B.rank = A.sched[2 * job + 1];
-        s_B.r0 = s_B.rank * s_B.D.rpc;
+        s_D = A.desc[inst];
+        s_rank = A.sched[2 * job + 1];
     }
     __syncthreads();
-    BlockCtx& B = s_B;
-    const InstanceDesc& D = B.D;
+    const InstanceDesc& D = s_D;
+    const int rank = s_rank, rep0 = rank * D.rpc;
     const int n = D.n, npad = D.n_pad, R = D.R, nt = D.nt, rpc = D.rpc, kst = D.kmax + 1;
 
     int32_t* s_col = sm_ptr<int32_t>(smem, S.col);
     int32_t* s_h = sm_ptr<int32_t>(smem, S.h);
     // acceptance thresholds: shared memory, or read through L1 (field_gather)
     uint32_t* s_thr_w = sm_ptr<uint32_t>(smem, S.thr);
-    const uint32_t* s_thr = S.field_gather ? A.thr + D.thr_off : s_thr_w;
+    const bool thr_global = SPACE == SP_LARGE || (SPACE == SP_ANY && S.field_gather);
+    const uint32_t* s_thr = thr_global ? A.thr + D.thr_off : s_thr_w;
     double* s_ptab = sm_ptr<double>(smem, S.ptab);
     uint32_t* s_order = sm_ptr<uint32_t>(smem, S.order);
     double* s_beta = sm_ptr<double>(smem, S.beta);
@@ -1589,13 +1788,16 @@ __global__ void __launch_bounds__((REPLAY || (BLOCKTEAM && !NARROW)) ? 1024 : kN
     uint32_t* s_xrand = sm_ptr<uint32_t>(smem, S.xrand);
     int* s_lvl = sm_ptr<int>(smem, S.xlevel);
     uint32_t* s_tmp = sm_ptr<uint32_t>(smem, S.xpos);
-    uint8_t* s_icm = ((S.state_global || S.field_gather) && !S.icm_split)
-                         ? A.icm_pool + (size_t)blockIdx.x * (size_t)A.icm_pool_stride
-                         : smem + S.icm;
+    uint8_t* const g_icm = A.icm_pool + (size_t)blockIdx.x * (size_t)A.icm_pool_stride;
+    uint8_t* s_icm = smem + S.icm;
+    if (SPACE == SP_ANY && (S.state_global || S.field_gather) && !S.icm_split) s_icm = g_icm;
     int* s_misc = sm_ptr<int>(smem, S.misc);
     long long* s_mag = sm_ptr<long long>(smem, S.mag);
-    long long* s_team_acc = sm_ptr<long long>(smem, S.misc + 64);
-    int* s_team_bc = sm_ptr<int>(smem, S.misc + 64 + 8 * 32);   // 2 ints per team
+    // a block team's keys (two per warp) and control words; warp teams use
+    // the first two control words of a place of their own
+    unsigned long long* s_team_keys = sm_ptr<unsigned long long>(smem, S.misc + 64);
+    int* s_team_ctl = sm_ptr<int>(smem, S.misc + 64 + 16 * 32);
+    int* s_warp_ctl = sm_ptr<int>(smem, S.misc + 64);
 
     const int32_t* g_row = A.row + D.row_off;
     const uint32_t* g_adj = A.adj + D.adj_off;
@@ -1622,24 +1824,30 @@ __global__ void __launch_bounds__((REPLAY || (BLOCKTEAM && !NARROW)) ? 1024 : kN
             if (ab) bulk_g2s(s_adj, g_adj, ab, mbar);
         }
     }
-    if (tid == 0) {
-        if (S.state_global) {
-            // replicas too large for shared memory work on their master copy
-            B.spin = A.spins + D.spin_off + (long long)B.r0 * D.n_pad;
-            B.field = A.fields + D.spin_off + (long long)B.r0 * D.n_pad;
-        } else {
-            B.spin = sm_ptr<int8_t>(smem, S.spin);
-            B.field = S.field_gather ? nullptr : sm_ptr<int32_t>(smem, S.field);
-        }
-        B.slot = sm_ptr<uint32_t>(smem, S.slot);
-        B.rslot = sm_ptr<uint32_t>(smem, S.rslot);
-        B.tb = sm_ptr<int32_t>(smem, S.rslot) + rpc;
-        B.E = sm_ptr<long long>(smem, S.E);
-        B.h = D.has_h ? s_h : nullptr;
-        B.row = staged ? sm_ptr<int32_t>(smem, S.row) : g_row;
-        B.adj = staged ? sm_ptr<uint32_t>(smem, S.adj) : g_adj;
+    if (SPACE == SP_SHARED && !staged) {
+        // (recorded above; the other blocks of the group see the abort)
+        __syncthreads();
+        continue;
     }
-    __syncthreads();
+    BlockCtx B{D, rank, rep0};
+    B.spin = sm_ptr<int8_t>(smem, S.spin);
+    B.field = SPACE == SP_LARGE || (SPACE == SP_ANY && S.field_gather) ? nullptr : sm_ptr<int32_t>(smem, S.field);
+    if (SPACE == SP_ANY && S.state_global) {
+        // replicas too large for shared memory work on their master copy
+        B.spin = A.spins + D.spin_off + (long long)rep0 * D.n_pad;
+        B.field = A.fields + D.spin_off + (long long)rep0 * D.n_pad;
+    }
+    B.slot = sm_ptr<uint32_t>(smem, S.slot);
+    B.rslot = sm_ptr<uint32_t>(smem, S.rslot);
+    B.tb = sm_ptr<int32_t>(smem, S.rslot) + rpc;
+    B.E = sm_ptr<long long>(smem, S.E);
+    B.h = D.has_h ? s_h : nullptr;
+    B.row = sm_ptr<int32_t>(smem, S.row);
+    B.adj = sm_ptr<uint32_t>(smem, S.adj);
+    if (SPACE == SP_LARGE || (SPACE != SP_SHARED && !staged)) {
+        B.row = g_row;
+        B.adj = g_adj;
+    }
     for (int i = tid; i <= D.ncolors; i += T) s_col[i] = A.col[D.col_off + i];
     if (D.has_h)
         for (int i = tid; i < n; i += T) s_h[i] = A.hpool[D.h_off + i];
@@ -1661,7 +1869,7 @@ __global__ void __launch_bounds__((REPLAY || (BLOCKTEAM && !NARROW)) ? 1024 : kN
         s_beta[k] = A.beta[D.beta_off + k];
     }
     for (int k = tid; k < nt * kst; k += T) {
-        if (!S.field_gather) s_thr_w[k] = A.thr[D.thr_off + k];
+        if (!thr_global) s_thr_w[k] = A.thr[D.thr_off + k];
         if (REPLAY) s_ptab[k] = A.ptab[D.ptab_off + k];
     }
     for (int j = tid; j < rpc; j += T) {
@@ -1676,10 +1884,7 @@ __global__ void __launch_bounds__((REPLAY || (BLOCKTEAM && !NARROW)) ? 1024 : kN
     unsigned int bar_gen = 0;
     if (tid == 0 && D.group > 1) bar_gen = *(volatile unsigned int*)(A.bar + 2 * inst + 1);
     if (tid == 0) {
-        for (int q = 0; q < 3; q++) team_slot_reset(s_team_acc, q);
-        s_team_bc[2] = 0;   // the block team's overlap-list and S counters
-        s_team_bc[3] = 0;
-        s_team_bc[4] = 0;
+        for (int q = 0; q < TC_WORDS; q++) s_team_ctl[q] = 0;
     }
     __syncthreads();
     for (int k = tid; k + 1 < nt; k += T) s_dbeta[k] = s_beta[k] - s_beta[k + 1];
@@ -1698,15 +1903,16 @@ __global__ void __launch_bounds__((REPLAY || (BLOCKTEAM && !NARROW)) ? 1024 : kN
     __syncthreads();
 
     const bool icm_on = (A.phase_mask & PHASE_ICM) && D.nc > 0 && D.chains >= 2;
-    Prof P;
-    P.init((A.prof != nullptr) && tid == 0, s_prof);
-    const long long t_start = P.mark;
+    const Prof P{A.prof != nullptr && tid == 0, &s_prof};
+    P.init();
+    const long long t_start = P.on ? s_prof.mark : 0;
     const bool best_pp = (A.flags & ENGINE_BEST_PER_PHASE) != 0;
     unsigned long long t_step1 = 0;
     for (int ls = 0; ls < A.nsteps; ls++) {
         if (ls == 1 && tid == 0) t_step1 = globaltimer_ns();
-        if (D.group == 1) {
-            // (a group of blocks sees an abort in its barrier)
+        if (D.group == 1 && (ls & 15) == 0) {
+            // (a group of blocks sees an abort in its barrier; a block alone
+            // looks every sixteenth step, a read of L2)
             if (tid == 0) s_misc[3] = *abortf;
             __syncthreads();
             if (s_misc[3]) break;
@@ -1729,7 +1935,7 @@ __global__ void __launch_bounds__((REPLAY || (BLOCKTEAM && !NARROW)) ? 1024 : kN
             }
         }
         P.tick(PROF_SWEEP);
-        if (cold) P.c[PROF_SWEEP_ICM] += clock64() - t_sw;
+        if (cold) s_prof.c[PROF_SWEEP_ICM] += clock64() - t_sw;
         const bool observe = A.obs != nullptr && D.hist_nbins > 0 && step >= A.hist_from;
         if (observe) {
             // magnetisation of the block's replicas, one warp per replica
@@ -1745,42 +1951,66 @@ __global__ void __launch_bounds__((REPLAY || (BLOCKTEAM && !NARROW)) ? 1024 : kN
                 for (int j = tid; j < rpc; j += T)
                     A.mag_pub[parity * A.energy_pub_half + D.rep_off + B.r0 + j] = s_mag[j];
         }
+        // the exchange's draws, before the wait for the energies
+        EvenOddDraws xdraw{0.f, 0.f};
+        const bool even_odd = !REPLAY && (A.phase_mask & PHASE_EXCHANGE) && (A.flags & ENGINE_EXCHANGE_EVEN_ODD);
+        // Publishes this block's spins (for ICM partners) as words of 32
+        // sites carrying the step's tag: a partner checks the tag of each
+        // word it reads, so nothing orders these stores and no fence waits
+        // for them (one bit a site: N=2000 goes out in 63 words).
+        // A thread packs the 32 spin bytes of a word: the sign bits of four
+        // bytes are gathered by one multiplication.
+        auto publish_spins = [&]() {
+            const int W = (n + 31) >> 5, npw = npad >> 4;
+            const unsigned long long tagw = (unsigned long long)(A.pub_base + (uint32_t)ls) << 32;
+            unsigned long long* const out = A.spins_pub + parity * A.spins_pub_half + (D.spin_off >> 4) + (long long)B.r0 * npw;
+            const int8_t* const sp = B.spin;
+            for (int j = 0; j < rpc; j++)
+                for (int k = tid; k < W; k += T) {
+                    const uint4* const q = reinterpret_cast<const uint4*>(sp + (long long)j * npad + 32 * k);
+                    uint32_t v[8] = {};
+                    const uint4 lo = q[0];
+                    v[0] = lo.x; v[1] = lo.y; v[2] = lo.z; v[3] = lo.w;
+                    if (32 * k + 16 < npad) {
+                        const uint4 hi = q[1];
+                        v[4] = hi.x; v[5] = hi.y; v[6] = hi.z; v[7] = hi.w;
+                    }
+                    uint32_t bits = 0;
+#pragma unroll
+                    for (int b = 0; b < 8; b++)
+                        bits |= ((((~v[b] >> 7) & 0x01010101u) * 0x10204080u) >> 28) << (4 * b);
+                    st_relaxed_gpu_u64(out + (long long)j * npw + k, tagw | bits);
+                }
+        };
         if (D.group > 1 && A.flag_barrier) {
-            // publish this block's spins (for ICM partners), then each of its
-            // replicas' energy tagged with this step in one 64-bit word,
-            // stored with release; wait for every other replica's word of
-            // this step, acquiring its block's spins with it.  No counter
-            // to arrive at and no second hop: a block goes on as soon as the
-            // last word it needs lands, holding the energies it read.
-            if (icm_on) {
-                const long long base = parity * A.spins_pub_half + D.spin_off + (long long)B.r0 * npad;
-                for (int idx = tid; idx < rpc * npad; idx += T) A.spins_pub[base + idx] = B.spin[idx];
-            }
-            __syncthreads();
+            // publish each of the block's replicas' energy tagged with this
+            // step in one 64-bit word, then its spins; wait for every other
+            // replica's word of this step.  Every word read across blocks
+            // carries its own tag, so the words need no order among
+            // themselves: a release and an acquire (two L2 round trips on
+            // the step's critical path) are paid only when published
+            // magnetisations, which carry no tag, ride along.
             unsigned long long* const ew = reinterpret_cast<unsigned long long*>(A.energy_pub) +
                                            (parity * A.energy_pub_half + D.rep_off) * kPubStride;
             const uint32_t tag = A.pub_base + (uint32_t)ls;
-            for (int j = tid; j < rpc; j += T)
-                st_release_gpu_u64(ew + (B.r0 + j) * kPubStride, pub_word(tag, B.E[B.r0 + j]));
+            if (observe) __syncthreads();
+            for (int j = tid; j < rpc; j += T) {
+                const unsigned long long w = pub_word(tag, B.E[B.r0 + j]);
+                if (observe) st_release_gpu_u64(ew + (B.r0 + j) * kPubStride, w);
+                else st_relaxed_gpu_u64(ew + (B.r0 + j) * kPubStride, w);
+            }
+            if (icm_on) publish_spins();
+            if (even_odd) xdraw = even_odd_draw(A, D, step);
             const unsigned long long limit = A.wait_limit_ns ? A.wait_limit_ns : kWaitLimitNs;
             int ok = 1;
             bool polled = false;
-            for (int r = tid; r < R && ok; r += T) {
-                if (r >= B.r0 && r < B.r0 + rpc) continue;
-                polled = true;
-                const unsigned long long t0 = globaltimer_ns();
-                unsigned int spins = 0;
-                unsigned long long w;
-                while ((uint32_t)((w = ld_relaxed_gpu_u64(ew + r * kPubStride)) >> 32) != tag) {
-                    if (*abortf) { ok = 0; break; }
-                    if ((++spins & 63u) == 0 && globaltimer_ns() - t0 > limit) {
-                        dev_fail(A.status, A.abort_flag, DEV_BARRIER_TIMEOUT, 1, blockIdx.x, tag);
-                        ok = 0;
-                        break;
-                    }
-                    __nanosleep(32);
-                }
-                if (ok) B.E[r] = (long long)(int32_t)(uint32_t)w;
+            for (int r0 = tid & ~31; r0 < R && ok; r0 += T) {
+                const int r = r0 + (tid & 31);
+                const bool need = r < R && (r < B.r0 || r >= B.r0 + rpc);
+                unsigned long long w = 0;
+                ok = poll_tagged(ew + (need ? r : 0) * kPubStride, need, tag, w, abortf, A.status, limit, 1);
+                if (need && ok) B.E[r] = (long long)(int32_t)(uint32_t)w;
+                polled |= need;
             }
             if (A.bar_phantom && tid == 0 && ok) {
                 // test hook: one more member whose word never comes
@@ -1793,23 +2023,21 @@ __global__ void __launch_bounds__((REPLAY || (BLOCKTEAM && !NARROW)) ? 1024 : kN
                     } else __nanosleep(256);
                 }
             }
-            // the words were read relaxed: each thread that read one acquires
-            // what its release published (the block's barrier passes it on)
-            if (polled) fence_acq_rel_gpu();
+            if (observe && polled) fence_acq_rel_gpu();
             if (!__syncthreads_and(ok)) break;
         } else if (D.group > 1) {
             // publish this block's energies (and spins, for ICM partners)
             for (int j = tid; j < rpc; j += T) A.energy_pub[parity * A.energy_pub_half + D.rep_off + B.r0 + j] = B.E[B.r0 + j];
-            if (icm_on) {
-                const long long base = parity * A.spins_pub_half + D.spin_off + (long long)B.r0 * npad;
-                for (int idx = tid; idx < rpc * npad; idx += T) A.spins_pub[base + idx] = B.spin[idx];
-            }
+            if (icm_on) publish_spins();
+            if (even_odd) xdraw = even_odd_draw(A, D, step);
             if (!group_barrier(A.bar + 2 * inst, (unsigned)(D.group + A.bar_phantom), abortf, A.status, bar_gen,
                                A.wait_limit_ns ? A.wait_limit_ns : kWaitLimitNs))
                 break;
             for (int r = tid; r < R; r += T)
                 if (r < B.r0 || r >= B.r0 + rpc) B.E[r] = ld_cg(A.energy_pub + parity * A.energy_pub_half + D.rep_off + r);
             __syncthreads();
+        } else if (even_odd) {
+            xdraw = even_odd_draw(A, D, step);
         }
         P.tick(PROF_BARRIER);
         if (A.hist != nullptr && D.hist_nbins > 0 && step >= A.hist_from && B.rank == 0) {
@@ -1831,7 +2059,7 @@ __global__ void __launch_bounds__((REPLAY || (BLOCKTEAM && !NARROW)) ? 1024 : kN
         }
         if (A.phase_mask & PHASE_EXCHANGE) {
             if (REPLAY) exchange_replay(A, B, ls, s_beta, s_att, s_succ);
-            else if (A.flags & ENGINE_EXCHANGE_EVEN_ODD) exchange_even_odd(A, B, step, s_dbeta, s_att, s_succ);
+            else if (A.flags & ENGINE_EXCHANGE_EVEN_ODD) exchange_even_odd(A, B, step, s_dbeta, s_att, s_succ, xdraw);
             else exchange_reference_order(A, B, step, s_order, s_dbeta, s_att, s_succ, s_xlogu, s_xrand, s_lvl, s_tmp, s_misc, P);
             for (int s = tid; s < R; s += T) {
                 const uint32_t r = B.slot[s];
@@ -1854,17 +2082,17 @@ __global__ void __launch_bounds__((REPLAY || (BLOCKTEAM && !NARROW)) ? 1024 : kN
             // the instance is configured with one team (large instances: a
             // pair per block-wide team, in sequence, beats a pair per warp)
             if (BLOCKTEAM || D.teams == 1) {
-                const Team<true> team{tid, T, s_team_acc, s_team_bc};
+                const Team<true> team{tid, T, s_team_ctl, s_team_keys};
                 IcmScratch X = icm_scratch(s_icm, npad);
-                if (!BLOCKTEAM && !REPLAY && S.icm_split)
-                    X.list = reinterpret_cast<int*>(A.icm_pool + (size_t)blockIdx.x * (size_t)A.icm_pool_stride);
+                if (SPACE == SP_LARGE || (SPACE == SP_ANY && !BLOCKTEAM && !REPLAY && S.icm_split))
+                    X.list = reinterpret_cast<int*>(g_icm);
                 for (int j = 0; j < rpc; j++) {
                     const int sl = (int)B.rslot[j], c = sl / nt, k = sl - c * nt, kk = nt - 1 - k;
                     if (kk >= D.nc || c >= chains_even) continue;
                     const int cp = c >> 1;
                     const int rA = (int)B.slot[(2 * cp) * nt + k], rB = (int)B.slot[(2 * cp + 1) * nt + k];
                     if ((c & 1) && rA >= B.r0 && rA < B.r0 + rpc) continue;
-                    icm_pair<true, REPLAY, !REPLAY && (NARROW || !BLOCKTEAM), !REPLAY && !BLOCKTEAM>(
+                    icm_pair<true, REPLAY, !REPLAY && (NARROW || !BLOCKTEAM), SPACE, !REPLAY && !BLOCKTEAM>(
                                                                              A, B, team, cp * D.nc + kk, rA, rB,
                                                                              step, ls, X, 30, P);
                 }
@@ -1872,7 +2100,7 @@ __global__ void __launch_bounds__((REPLAY || (BLOCKTEAM && !NARROW)) ? 1024 : kN
                 const int warp = tid >> 5, lane = tid & 31;
                 const int teams = min(D.teams, T >> 5);
                 if (warp < teams) {
-                    Team<false> team{lane, 32, s_team_acc + warp, s_team_bc + 2 * warp};
+                    const Team<false> team{lane, 32, s_warp_ctl + 2 * warp, nullptr};
                     const IcmScratch X = icm_scratch(s_icm + (size_t)warp * icm_team_bytes(npad), npad);
                     int e = 0;
                     for (int j = 0; j < rpc; j++) {
@@ -1882,23 +2110,19 @@ __global__ void __launch_bounds__((REPLAY || (BLOCKTEAM && !NARROW)) ? 1024 : kN
                         const int rA = (int)B.slot[(2 * cp) * nt + k], rB = (int)B.slot[(2 * cp + 1) * nt + k];
                         if ((c & 1) && rA >= B.r0 && rA < B.r0 + rpc) continue;
                         if ((e++ % teams) != warp) continue;
-                        icm_pair<false, REPLAY, false>(A, B, team, cp * D.nc + kk, rA, rB, step, ls, X, 30, P);
+                        icm_pair<false, REPLAY, false, SPACE>(A, B, team, cp * D.nc + kk, rA, rB, step, ls, X, 30, P);
                     }
                 }
             }
             __syncthreads();
-            // the block team's reduction slots back to the identity (the
-            // next step's barriers publish it)
-            if (tid == 0)
-                for (int q = 0; q < 3; q++) team_slot_reset(s_team_acc, q);
         }
         P.tick(PROF_ICM);
     }
     __syncthreads();
     if (A.job_ns != nullptr && tid == 0 && A.nsteps > 1) A.job_ns[job] = globaltimer_ns() - t_step1;
     if (P.on) {
-        P.c[PROF_TOTAL] = clock64() - t_start;
-        for (int q = 0; q < PROF_PHASES; q++) A.prof[(size_t)blockIdx.x * PROF_PHASES + q] += (unsigned long long)P.c[q];
+        s_prof.c[PROF_TOTAL] = clock64() - t_start;
+        for (int q = 0; q < PROF_PHASES; q++) A.prof[(size_t)blockIdx.x * PROF_PHASES + q] += (unsigned long long)s_prof.c[q];
     }
     // ---- write the block's state back
     if (!S.state_global) {
@@ -2070,11 +2294,23 @@ __global__ void evaluate_kernel(const int32_t* row, const uint32_t* adj, const i
 }
 
 // ------------------------------------------------------------ launchers
-static void* engine_fn(bool replay, bool block_team, bool narrow) {
-    if (replay) return (void*)pt_engine_kernel<true, false, false>;
-    if (block_team && narrow) return (void*)pt_engine_kernel<false, true, true>;
-    if (block_team) return (void*)pt_engine_kernel<false, true, false>;
-    return (void*)pt_engine_kernel<false, false, false>;
+static void* engine_fn(bool replay, bool block_team, bool narrow, int space) {
+    if (replay) return (void*)pt_engine_kernel<true, false, false, SP_ANY>;
+    if (block_team && narrow)
+        return space == SP_SHARED ? (void*)pt_engine_kernel<false, true, true, SP_SHARED>
+                                  : (void*)pt_engine_kernel<false, true, true, SP_ANY>;
+    if (block_team) return (void*)pt_engine_kernel<false, true, false, SP_ANY>;
+    if (space == SP_SHARED || space == SP_STATE) return (void*)pt_engine_kernel<false, false, false, SP_STATE>;
+    if (space == SP_LARGE) return (void*)pt_engine_kernel<false, false, false, SP_LARGE>;
+    return (void*)pt_engine_kernel<false, false, false, SP_ANY>;
+}
+
+// The address spaces of a plan's launch.  (A staged plan of one instance
+// stages that instance; a batch stages some of its instances.)
+static int plan_space(const SmemPlan& S, bool block_team) {
+    if (!S.state_global && !S.field_gather) return S.stage_adj && block_team ? SP_SHARED : SP_STATE;
+    if (S.field_gather && S.icm_split) return SP_LARGE;
+    return SP_ANY;
 }
 
 // Tags of published energy words: one per PT step of every launch in the
@@ -2083,7 +2319,7 @@ static std::atomic<uint32_t> g_pub_tag{1u};
 
 cudaError_t launch_engine(const EngineArgs& A0, int threads, bool replay, bool block_team, bool narrow,
                           bool cooperative, cudaStream_t stream) {
-    void* fn = engine_fn(replay, block_team, narrow);
+    void* fn = engine_fn(replay, block_team, narrow, plan_space(A0.sm, block_team));
     cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)A0.sm.total);
     if (e != cudaSuccess) return e;
     EngineArgs A = A0;
@@ -2102,10 +2338,17 @@ cudaError_t engine_max_blocks_per_sm(bool replay, bool block_team, bool narrow, 
         *out = 0;
         return cudaSuccess;
     }
-    const void* fn = engine_fn(replay, block_team, narrow);
-    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(out, fn, threads, smem);
+    // the launch takes one of the variants by its plan: what all of them hold
+    *out = 1 << 20;
+    for (int space : {SP_ANY, SP_SHARED, SP_STATE, SP_LARGE}) {
+        const void* fn = engine_fn(replay, block_team, narrow, space);
+        cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        int per_sm = 0;
+        if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, smem);
+        if (e != cudaSuccess) return e;
+        *out = std::min(*out, per_sm);
+    }
+    return cudaSuccess;
 }
 
 cudaError_t launch_recompute(const EngineArgs& A, const int32_t* rep_inst, int total_reps, int write_back,

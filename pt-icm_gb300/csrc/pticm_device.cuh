@@ -186,7 +186,6 @@ __device__ __forceinline__ uint32_t bounded32(uint32_t x, uint32_t range) {
 
 // ---------------------------------------------------- cross-block memory
 __device__ __forceinline__ long long ld_cg(const long long* p) { return __ldcg(p); }
-__device__ __forceinline__ int8_t ld_cg(const int8_t* p) { return (int8_t)__ldcg((const signed char*)p); }
 
 // -------------------------------------------------------- group barrier
 __device__ __forceinline__ unsigned int ld_acquire_gpu(const unsigned int* p) {
@@ -217,6 +216,44 @@ __device__ __forceinline__ void fence_acq_rel_gpu() {
 
 __device__ __forceinline__ void st_release_gpu_u64(unsigned long long* p, unsigned long long v) {
     asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
+
+__device__ __forceinline__ void st_relaxed_gpu_u64(unsigned long long* p, unsigned long long v) {
+    asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
+
+// A warp polls one published word per lane (`need`: this lane waits for one)
+// until the high half of each is `tag`; false when the limit ran out or
+// another block raised `abort`, both looked at by one lane every 64th poll
+// (every thread reading the one abort word queues on its L2 line: with the
+// 65536 pollers of the large instance 60 us a time).  The pause between
+// polls grows with the wait: polls without one keep L2 busy and slow the
+// blocks still working.
+__device__ __forceinline__ bool poll_tagged(const unsigned long long* p, bool need, uint32_t tag, unsigned long long& w,
+                                            volatile int* abort_flag, DevStatus* st, unsigned long long limit_ns,
+                                            int where) {
+    unsigned long long t0 = 0;
+    for (unsigned int spins = 1;; spins++) {
+        if (need) {
+            w = ld_relaxed_gpu_u64(p);
+            need = (uint32_t)(w >> 32) != tag;
+        }
+        if (!__any_sync(0xffffffffu, need)) return true;
+        if ((spins & 63u) == 0) {
+            int stop = 0;
+            if ((threadIdx.x & 31) == 0) {
+                const unsigned long long t = globaltimer_ns();
+                if (t0 == 0) t0 = t;
+                if (*abort_flag) stop = 1;
+                else if (t - t0 > limit_ns) {
+                    dev_fail(st, abort_flag, DEV_BARRIER_TIMEOUT, where, blockIdx.x, tag);
+                    stop = 1;
+                }
+            }
+            if (__shfl_sync(0xffffffffu, stop, 0)) return false;
+        }
+        __nanosleep(spins < 32u ? 32u : 256u);
+    }
 }
 
 // A replica's published energy word: the publishing step's tag in the high

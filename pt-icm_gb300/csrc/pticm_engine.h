@@ -112,8 +112,11 @@ struct EngineArgs {
     int8_t* spins;                // master copy
     int32_t* fields;
     long long* energy;
-    int8_t* spins_pub;            // 2 halves, parity of the PT step
-    long long spins_pub_half;     // elements per half
+    // published spins, 2 halves by the parity of the PT step: a replica's
+    // sites 32 k .. 32 k + 31 are one word, tag << 32 | a bit per site (set:
+    // +1), at (spin offset of the replica) / 16 + k
+    unsigned long long* spins_pub;
+    long long spins_pub_half;     // words per half (spin pool size / 16)
     long long* energy_pub;        // 2 * total replicas (x kPubStride words with flag_barrier)
     long long energy_pub_half;
     unsigned long long* flips;
@@ -170,6 +173,9 @@ struct EngineArgs {
     // pub_base + (step within the launch) is the tag; launch_engine sets it.
     int32_t flag_barrier;
     uint32_t pub_base;
+    // every energy lies in (-2^30, 2^30): energy changes and sums are exact
+    // modulo 2^32
+    int32_t small_energy;
 };
 
 enum EngineFlags : int32_t {

@@ -91,7 +91,8 @@ struct pticm_ctx {
     DArr<int32_t> d_sched_off, d_sched, d_rep_inst, d_row, d_col, d_h, d_perm;
     DArr<uint32_t> d_adj, d_thr, d_slot, d_order, d_cursor;
     DArr<double> d_beta, d_ptab;
-    DArr<int8_t> d_spins, d_pub, d_best_state;
+    DArr<int8_t> d_spins, d_best_state;
+    DArr<unsigned long long> d_pub;   // published spin words (two halves)
     DArr<int32_t> d_fields;
     DArr<long long> d_E, d_Epub, d_bestE;
     DArr<unsigned long long> d_flips, d_bestSweep, d_att, d_succ, d_mismatch, d_prof;
@@ -543,7 +544,7 @@ EngineArgs make_args(pticm_ctx* c) {
     A.fields = c->d_fields.p;
     A.energy = c->d_E.p;
     A.spins_pub = c->d_pub.p;
-    A.spins_pub_half = (long long)c->R * c->desc.n_pad;
+    A.spins_pub_half = (long long)c->R * c->desc.n_pad / 16;
     A.energy_pub = c->d_Epub.p;
     A.energy_pub_half = c->R;
     A.flips = c->d_flips.p;
@@ -573,6 +574,7 @@ EngineArgs make_args(pticm_ctx* c) {
     A.bar_phantom = c->bar_phantom;
     if (c->ebound < 0) c->ebound = energy_bound(c->P);
     A.flag_barrier = c->ebound < (1ll << 31) ? 1 : 0;   // every energy fits the word's 32 bits
+    A.small_energy = c->ebound < (1ll << 30) ? 1 : 0;
     return A;
 }
 
@@ -983,7 +985,7 @@ int pticm_create(const pticm_problem* p, const pticm_opts* o, pticm_ctx** out) {
     CK(c->d_spins.alloc(spins));
     CK(c->d_fields.alloc(spins));
     CK(c->d_best_state.alloc(spins));
-    CK(c->d_pub.alloc(2 * spins));
+    CK(c->d_pub.alloc(2 * (spins / 16)));
     CK(c->d_E.alloc(c->R));
     CK(c->d_Epub.alloc(2 * c->R * kPubStride));
     CK(c->d_bestE.alloc(c->R));
