@@ -15,7 +15,8 @@ struct MhJob {
     int64_t bin0;
     double min_emin;
     double estep;
-    double logn;
+    double n;      // samples
+    double logn;   // ln n
 };
 
 }  // namespace pticm

@@ -630,9 +630,11 @@ int reset_run_state(pticm_ctx* c) {
 }  // namespace
 
 namespace pticm {
-cudaError_t mhist_solve(const MhJob* jobs, int njobs, int max_nt, const uint32_t* hist, const uint64_t* hoff,
+cudaError_t mhist_plan(const std::vector<MhJob>& jobs, int max_nt, int& cs, size_t& bytes, std::vector<long long>& off);
+cudaError_t mhist_solve(int njobs, int cs, const MhJob* jobs, const uint32_t* hist, const uint64_t* hoff,
                         const uint64_t* hlen, const double* emin, const double* beta, double* logdos, double* logc,
-                        float* ldf, double* logZ, unsigned long long* iters, long long max_iters, cudaStream_t st);
+                        float* ldf, double* logZ, unsigned long long* iters, long long max_iters, uint8_t* work,
+                        const long long* work_off, cudaStream_t st);
 }  // namespace pticm
 
 namespace pticm {
@@ -670,6 +672,7 @@ int mhist_dos_multi(const std::vector<const MhInput*>& in, std::vector<MhOutput>
         J.bin0 = bins;
         J.min_emin = me;
         J.estep = I.estep;
+        J.n = (double)I.n;
         J.logn = std::log((double)I.n);
         const uint64_t base = hist.size();
         hist.insert(hist.end(), I.hist.begin(), I.hist.end());
@@ -691,6 +694,14 @@ int mhist_dos_multi(const std::vector<const MhInput*>& in, std::vector<MhOutput>
     DArr<unsigned long long> d_it;
     DArr<double> d_emin, d_beta, d_logZ, d_dos, d_logc;
     DArr<float> d_ldf;
+    DArr<uint8_t> d_work;
+    DArr<long long> d_work_off;
+    std::vector<long long> work_off;
+    int cs = 1;
+    size_t work_bytes = 0;
+    CK(mhist_plan(jobs, max_nt, cs, work_bytes, work_off));
+    CK(d_work.alloc(work_bytes));
+    CK(d_work_off.upload(work_off));
     CK(d_jobs.upload(jobs));
     CK(d_hist.upload(hist, 1));
     CK(d_off.upload(hoff));
@@ -702,8 +713,8 @@ int mhist_dos_multi(const std::vector<const MhInput*>& in, std::vector<MhOutput>
     CK(d_logc.alloc((size_t)bins));
     CK(d_ldf.alloc((size_t)bins));
     CK(d_it.alloc(jobs.size()));
-    CK(mhist_solve(d_jobs.p, (int)jobs.size(), max_nt, d_hist.p, d_off.p, d_len.p, d_emin.p, d_beta.p, d_dos.p,
-                   d_logc.p, d_ldf.p, d_logZ.p, d_it.p, kMhistMaxIters, nullptr));
+    CK(mhist_solve((int)jobs.size(), cs, d_jobs.p, d_hist.p, d_off.p, d_len.p, d_emin.p, d_beta.p, d_dos.p,
+                   d_logc.p, d_ldf.p, d_logZ.p, d_it.p, kMhistMaxIters, d_work.p, d_work_off.p, nullptr));
     CK(cudaDeviceSynchronize());
     std::vector<double> dos, z;
     std::vector<unsigned long long> it;
