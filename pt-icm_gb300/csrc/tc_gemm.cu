@@ -26,6 +26,7 @@
 #include <cstdint>
 
 #include "pticm_device.cuh"
+#include "tc_device.cuh"
 
 namespace pticm {
 
@@ -44,17 +45,6 @@ __device__ __forceinline__ uint64_t tc_smem_desc(uint32_t saddr, uint32_t lbo, u
     d |= (uint64_t)1 << 46;
     return d;
 }
-
-// Instruction descriptor of kind::f16: FP32 accumulator, BF16 A and B, both
-// K-major, N >> 3 at bit 17, M >> 4 at bit 24.
-__host__ __device__ constexpr uint32_t tc_idesc_bf16(int M, int N) {
-    return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
-}
-
-__device__ __forceinline__ void tc_fence_proxy_async() {
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-}
-
 
 // Epilogue of one accumulator row segment: 32 FP32 columns from cb on,
 // plus bias, stored as FP32 (pre-activation) and/or BF16 (after the
@@ -270,16 +260,6 @@ tc_gemm_kernel(const __nv_bfloat16* __restrict__ A, const __nv_bfloat16* __restr
 // 128-byte atoms 1024 bytes apart, each K=16 step 32 bytes further into the
 // atom.  Stage buffers start on 1024 bytes.
 constexpr int TC_TMA_STAGES = 4;
-
-__device__ __forceinline__ uint64_t tc_smem_desc_sw128(uint32_t saddr) {
-    uint64_t d = 0;
-    d |= (uint64_t)((saddr >> 4) & 0x3FFFu);
-    d |= (uint64_t)1 << 16;              // leading byte offset (unused for swizzled K-major)
-    d |= (uint64_t)(1024 >> 4) << 32;    // stride byte offset: 8-row atoms 1024 B apart
-    d |= (uint64_t)1 << 46;              // descriptor version
-    d |= (uint64_t)2 << 61;              // SWIZZLE_128B
-    return d;
-}
 
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
     asm volatile(
