@@ -1159,6 +1159,35 @@ __device__ __forceinline__ int gather_field(const int32_t* row, const uint32_t* 
     return f;
 }
 
+// The part of site i's local field that thread `sub` of G gathers: the 16-byte
+// pieces sub, sub + G, ... of its neighbour list, two at a time, entries
+// outside the list as zeros.  All loads of a pair of pieces are independent;
+// a list walked entry by entry up to alignment and from there takes twice as
+// long as its twenty neighbours' loads (N=2000: 0.93 us a colour class).
+// (The list starts on 16 bytes and is readable to the end of its last piece.)
+__device__ __forceinline__ int gather_pieces(const int32_t* row, const uint32_t* adj, const int8_t* sp, int i, int sub,
+                                             int G) {
+    const int e0 = row[i], deg = row[i + 1] - e0, p1 = (e0 + deg + 3) >> 2;
+    const uint4* const adj4 = reinterpret_cast<const uint4*>(adj);
+    int f = 0;
+    for (int p = (e0 >> 2) + sub; p < p1; p += 2 * G) {
+        const uint4 u = adj4[p];
+        uint4 v = make_uint4(0, 0, 0, 0);
+        if (p + G < p1) v = adj4[p + G];
+        uint32_t e[8] = {u.x, u.y, u.z, u.w, v.x, v.y, v.z, v.w};
+        int s[8];
+#pragma unroll
+        for (int k = 0; k < 8; k++) {
+            const int at = 4 * (k < 4 ? p : p + G) + (k & 3);
+            if ((unsigned)(at - e0) >= (unsigned)deg) e[k] = 0;
+            s[k] = sp[e[k] >> 8];
+        }
+#pragma unroll
+        for (int k = 0; k < 8; k++) f += (int)(int8_t)(e[k] & 0xffu) * s[k];
+    }
+    return f;
+}
+
 // --------------------------------------------------------------- sweeps
 // A warp pushes the field changes of at most this many accepted sites one
 // site at a time (a lane per neighbour); with more, each lane pushes its own
@@ -1172,10 +1201,12 @@ constexpr int kGatherReps = 4;
 // Colour-class Metropolis sweep of the block's replicas (production).
 // dE_i = -2 s_i (h_i + f_i); accepted with probability min(1, exp(-beta dE))
 // (src/replica.cc:31-38); an accepted flip pushes J_ij * (-2 s_i) into each
-// neighbour's field (the integer form of src/problem.cc:164-181).  With one
-// replica per block (ONE) every thread keeps its energy change and flip
-// count in registers until a phase boundary; with several, warps aggregate
-// per replica before touching shared memory.
+// neighbour's field (the integer form of src/problem.cc:164-181), or, where no
+// fields are stored, every visit gathers its own.  With one replica per block
+// (ONE) every thread keeps its energy change and flip count in registers until
+// a phase boundary; with several, warps aggregate per replica before touching
+// shared memory.  COOP: the narrow block team, whose instances with few
+// neighbours gather (InstanceDesc::lanes), and whose others push together.
 template <bool ONE, bool COOP>
 __device__ void colored_sweep(const EngineArgs& A, const BlockCtx& B, unsigned long long sweep_idx,
                               int32_t* s_col, const uint32_t* s_thr, int* s_dEp, unsigned* s_flp,
@@ -1190,7 +1221,10 @@ __device__ void colored_sweep(const EngineArgs& A, const BlockCtx& B, unsigned l
     ThreadRng12 rng;
     // counter: (rank in the group, thread), sweep, instance id in the high
     // half of the call word (a thread makes far fewer than 2^16 calls)
-    rng.start(stream_key(A.seed, STREAM_SWEEP), (uint32_t)(B.rank * T + tid), sweep_idx, (uint32_t)D.inst_id << 16);
+    const int G = ONE && COOP ? D.lanes : 0, ng = G > 0 ? T / G : T, grp = G > 0 ? tid / G : tid,
+              sub = G > 0 ? tid & (G - 1) : 0;
+    rng.start(stream_key(A.seed, STREAM_SWEEP), (uint32_t)(B.rank * T + grp + sub * ng), sweep_idx,
+              (uint32_t)D.inst_id << 16);
     int acc_de = 0;
     unsigned acc_fl = 0;
     // several replicas in the block, fields gathered
@@ -1254,6 +1288,39 @@ __device__ void colored_sweep(const EngineArgs& A, const BlockCtx& B, unsigned l
                     }
                 }
             }
+        } else if (ONE && COOP && G > 0) {
+            // A site's field is gathered by G neighbouring threads (no stored
+            // fields: nothing to push, so hot and cold replicas cost alike).
+            // Every thread keeps the random stream of one of the T logical
+            // threads that the sites of a class are dealt to: thread g G + s
+            // that of logical thread g + s T / G, so that a class of at most
+            // T / G sites uses all threads, and a larger one takes its
+            // T / G-site portions in turn.
+            for (int j0 = 0; j0 < Sc; j0 += T)
+                for (int s = 0; s < G; s++) {
+                    const int portion = j0 + s * ng;
+                    if (portion >= Sc) break;
+                    const int j = portion + grp, i = c0 + j;
+                    const bool have = j < Sc, mine = have && sub == s;
+                    if (mine) rng.fill_one();   // (runs under the gather's loads)
+                    int f = 0;
+                    if (have) f = gather_pieces(row, adj, sp1, i, sub, G);
+                    for (int o = G >> 1; o > 0; o >>= 1) f += __shfl_xor_sync(0xffffffffu, f, o);
+                    if (mine) {
+                        const int sv = sp1[i];
+                        const int de = -2 * sv * (f + (h1 != nullptr ? h1[i] : 0));
+                        bool acc = de <= 0;
+                        if (!acc) {
+                            const uint32_t thr = thr1[min(de >> 1, kmax)];
+                            acc = (rng.next_one() < thr) || (thr == 0xFFFFFFFFu);
+                        }
+                        if (acc) {
+                            sp1[i] = (int8_t)-sv;
+                            acc_de += de;
+                            acc_fl++;
+                        }
+                    }
+                }
         } else if (ONE) {
             int8_t* sp = B.spin;
             int32_t* fd = B.field;   // null in field_gather mode
@@ -1831,11 +1898,12 @@ __global__ void __launch_bounds__((REPLAY || (BLOCKTEAM && !NARROW)) ? 1024 : kN
     }
     BlockCtx B{D, rank, rep0};
     B.spin = sm_ptr<int8_t>(smem, S.spin);
-    B.field = SPACE == SP_LARGE || (SPACE == SP_ANY && S.field_gather) ? nullptr : sm_ptr<int32_t>(smem, S.field);
+    // (a narrow block team with lanes gathers its fields)
+    B.field = (BLOCKTEAM && NARROW && D.lanes > 0) || SPACE == SP_LARGE || (SPACE == SP_ANY && S.field_gather) ? nullptr : sm_ptr<int32_t>(smem, S.field);
     if (SPACE == SP_ANY && S.state_global) {
         // replicas too large for shared memory work on their master copy
         B.spin = A.spins + D.spin_off + (long long)rep0 * D.n_pad;
-        B.field = A.fields + D.spin_off + (long long)rep0 * D.n_pad;
+        if (!(BLOCKTEAM && NARROW && D.lanes > 0)) B.field = A.fields + D.spin_off + (long long)rep0 * D.n_pad;
     }
     B.slot = sm_ptr<uint32_t>(smem, S.slot);
     B.rslot = sm_ptr<uint32_t>(smem, S.rslot);
@@ -2125,18 +2193,17 @@ __global__ void __launch_bounds__((REPLAY || (BLOCKTEAM && !NARROW)) ? 1024 : kN
         for (int q = 0; q < PROF_PHASES; q++) A.prof[(size_t)blockIdx.x * PROF_PHASES + q] += (unsigned long long)s_prof.c[q];
     }
     // ---- write the block's state back
-    if (!S.state_global) {
-        const long long base = D.spin_off + (long long)B.r0 * npad;
+    const long long base = D.spin_off + (long long)B.r0 * npad;
+    if (SPACE != SP_ANY || !S.state_global)
         for (int idx = tid; idx < rpc * npad; idx += T) {
             A.spins[base + idx] = B.spin[idx];
             if (B.field) A.fields[base + idx] = B.field[idx];
         }
-        if (S.field_gather) {
-            // the stored fields of the master copy, gathered once per launch
-            for (int idx = tid; idx < rpc * npad; idx += T) {
-                const int j = idx / npad, i = idx - j * npad;
-                A.fields[base + idx] = i < n ? gather_field(B.row, B.adj, B.spin + (long long)j * npad, i) : 0;
-            }
+    if (!B.field) {
+        // the stored fields of the master copy, gathered once per launch
+        for (int idx = tid; idx < rpc * npad; idx += T) {
+            const int j = idx / npad, i = idx - j * npad;
+            A.fields[base + idx] = i < n ? gather_field(B.row, B.adj, B.spin + (long long)j * npad, i) : 0;
         }
     }
     for (int j = tid; j < rpc; j += T) {

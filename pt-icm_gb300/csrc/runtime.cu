@@ -450,7 +450,43 @@ void single_instance_schedule(int group, std::vector<int32_t>& sched_off, std::v
     }
 }
 
+// How a narrow block team's sweep gets its fields.  Gathered by G threads per
+// site (G > 0): hot and cold replicas cost alike, and a hot replica's sweep is
+// much shorter (N=1500, degree 40: 46.7 -> 24.4 us, step 48.5 -> 36.9).  From
+// stored fields, updated by pushing accepted flips (0): a cold replica's sweep
+// is shorter from about degree 10 on, and with ICM the cold replicas' sweep
+// and pair are the step's critical path (N=2000, degree 20: step 21.2 against
+// 23.6 us gathered; degree 8: equal on 1000 sites, 1.03 times slower on 3500;
+// degree 6: 1.07 times slower; degree 30: 1.09 times faster; from degree 34 or
+// so the hot replicas' pushes are the critical path).  Lists in device memory
+// are gathered only for few neighbours (N=4541, degree 38: 1.13 times slower).
+constexpr double kGatherUpTo = 8.5, kGatherFrom = 34.0;
+
+// Threads per site: G threads share a list of `pieces` 16-byte pieces, a class
+// of S sites takes ceil(S G / threads) portions; a portion costs about 250
+// cycles, 110 per pair of pieces and 100 per halving of the list.
+static int gather_lanes(const HostProblem& P, int threads) {
+    const double pieces = (double)P.dadj.size() / (4.0 * (double)std::max<int64_t>(P.n, 1)) + 0.75;
+    int best = 1;
+    double best_cost = DBL_MAX;
+    for (int G = 1, lg = 0; G <= 32; G *= 2, lg++) {
+        const double portion = 250.0 + 100.0 * lg + 110.0 * std::ceil(pieces / (2 * G));
+        double cost = 0;
+        for (int k = 0; k < P.ncolors; k++)
+            cost += portion * std::ceil((double)(P.color_off[k + 1] - P.color_off[k]) * G / threads);
+        if (cost < best_cost) {
+            best_cost = cost;
+            best = G;
+        }
+    }
+    return best;
+}
+
 void finish_desc(InstanceDesc& D, const HostProblem& P, const pticm_opts& o, const LaunchConfig& cfg) {
+    const double degree = (double)P.dadj.size() / (double)std::max<int64_t>(P.n, 1);
+    const bool gather = cfg.narrow && (degree <= kGatherUpTo || cfg.field_gather ||
+                                       (cfg.plan.stage_adj && (D.nc == 0 || degree >= kGatherFrom)));
+    D.lanes = gather ? gather_lanes(P, cfg.threads) : 0;
     D.icm_algo = engine_flags(P, o) & ENGINE_ICM_MASK;
     D.stage = cfg.plan.stage_adj;
     D.rpc = cfg.rpc;
