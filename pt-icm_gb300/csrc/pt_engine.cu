@@ -1577,29 +1577,44 @@ __device__ void replay_sweep(const EngineArgs& A, const BlockCtx& B, int ls, int
 }
 
 // ------------------------------------------------------------- exchange
+// Accepts a swap with energy difference dE across dbeta: x = dbeta * dE > 0
+// or log u < x, in FP64.  The sign of x is the product of the signs, and the
+// comparison is decided in FP32 unless log u lies within 1e-5 of x relative
+// to |x| (the FP32 product is within 2^-21 of x), so that the FP64 pipe,
+// slow on this chip, is left to about one attempt in 10^5.
+__device__ __forceinline__ bool swap_accepted(double dbeta, long long dE, float log_u) {
+    const float db = (float)dbeta, xf = db * (float)dE;
+    if (dE == 0 && fabsf(db) < 1e30f) return log_u < 0.f;
+    if (fabsf(xf) > 1e-30f && fabsf(db) > 1e-30f) {
+        if (xf > 0.f) return true;
+        if (fabsf(log_u - xf) > 1e-5f * fabsf(xf)) return log_u < xf;
+    }
+    const double x = dbeta * (double)dE;
+    return x > 0.0 || (double)log_u < x;
+}
+
 // Production exchange with the reference's attempt order
 // (src/replica_exchange.cc:5-100): a shuffled order of the nt-1 adjacent
 // pairs is walked by one cursor shared by all chains (attempt a goes to chain
 // a % chains); the order is reshuffled whenever the cursor wraps.  Attempt
 // on pair k accepts iff dBeta*dE > 0 or log u < dBeta*dE, and swaps the
 // slot->replica entries.  Within one pass over the order each pair appears
-// once, so an attempt depends only on earlier attempts on the neighbouring
-// pairs of its chain: attempts are grouped into dependency levels and each
-// level runs in parallel, with exactly the sequential semantics.
-__device__ void exchange_reference_order(const EngineArgs& A, const BlockCtx& B, unsigned long long step,
-                                         uint32_t* s_order, const double* s_dbeta, unsigned* s_att,
-                                         unsigned* s_succ, float* s_xlogu, uint32_t* s_xrand,
-                                         int* s_lvl, uint32_t* s_tmp, int* s_misc, const Prof P) {
-    P.subtick(PROF_X_SHUFFLE);
-    const InstanceDesc& D = B.D;
-    const int tid = threadIdx.x, T = blockDim.x;
-    const int nt = D.nt, C = D.chains, m = nt - 1;
-    if (m <= 0) return;
-    const int total = C * m;
-    // pre-draw: total log-uniforms and total shuffle keys
+// once, so an attempt waits only for earlier attempts on the neighbouring
+// pairs of its chain; all attempts that wait for none are made together,
+// with exactly the sequential semantics.
+//
+// Everything but the energies is known beforehand: the draws (by the whole
+// block), and by one warp each pass's chains, waits and the next pass's order,
+// one word per (pass, pair), before the wait for the other blocks' energies.
+// (Levels by relaxation, attempts in FP64 and the reshuffles after that wait
+// took 8.2 us for 20 pairs and two chains.)
+constexpr uint32_t kWaitLeft = 1u << 30, kWaitRight = 1u << 31, kPosBits = 24;
+
+__device__ void exchange_reference_draw(const EngineArgs& A, const InstanceDesc& D, unsigned long long step,
+                                        float* s_xlogu, uint32_t* s_xrand) {
+    const int total = D.chains * (D.nt - 1), ndraw = 2 * total;
     const uint2 key = stream_key(A.seed, STREAM_EXCHANGE);
-    const int ndraw = 2 * total;
-    for (int call = tid; call * 4 < ndraw; call += T) {
+    for (int call = threadIdx.x; call * 4 < ndraw; call += blockDim.x) {
         const uint4 r = philox4x32_10(make_uint4((uint32_t)call, (uint32_t)D.inst_id, (uint32_t)step,
                                                  (uint32_t)(step >> 32)), key);
         const uint32_t v[4] = {r.x, r.y, r.z, r.w};
@@ -1611,80 +1626,127 @@ __device__ void exchange_reference_order(const EngineArgs& A, const BlockCtx& B,
         }
     }
     __syncthreads();
-    P.subtick(PROF_X_DRAW);
-    // one warp walks the rounds; the rest of the block waits at the end
-    if (tid < 32) {
-        const int lane = tid;
-        for (int round = 0; round < C; round++) {
-            // level of attempt i = 1 + max level of earlier attempts on the
-            // neighbouring pairs of the same chain
-            for (int i = lane; i < m; i += 32) {
-                s_lvl[i] = 1;
-                s_tmp[s_order[i]] = (uint32_t)i;   // position of each pair in this pass
+}
+
+// One warp: s_xrand's shuffle keys become, per (pass, pair), the pair's
+// position in the pass's order (low 24 bits), its chain (six bits) and whether
+// an earlier attempt on the pair below or above goes to the same chain.
+// s_pos: each pair's position after all passes' reshuffles, which the exchange
+// makes the order.
+__device__ void exchange_reference_plan(const InstanceDesc& D, const uint32_t* s_order, uint32_t* s_xrand,
+                                        uint32_t* s_pos, int* s_next) {
+    const int lane = threadIdx.x & 31, C = D.chains, m = D.nt - 1;
+    for (int i = lane; i < m; i += 32) s_pos[s_order[i]] = (uint32_t)i;
+    __syncwarp();
+    for (int round = 0; round < C; round++) {
+        uint32_t* const keys = s_xrand + round * m;
+        for (int kb = lane; kb < m; kb += 32) {
+            const int p = (int)s_pos[kb];
+            // the pair's next position: the rank of its key (ties by position)
+            const uint32_t mine = keys[p];
+            int rank = 0;
+#pragma unroll 8
+            for (int j = 0; j < m; j++) {
+                const uint32_t kj = keys[j];
+                rank += (kj < mine) || (kj == mine && j < p);
             }
-            __syncwarp();
-            for (int iter = 0; iter <= m; iter++) {
-                int changed = 0;
-                for (int i = lane; i < m; i += 32) {
-                    const int kb = (int)s_order[i];
-                    const int c = (round * m + i) % C;
-                    int lv = 1;
-                    if (kb > 0) {
-                        const int jn = (int)s_tmp[kb - 1];
-                        if (jn < i && (round * m + jn) % C == c) lv = max(lv, ((volatile int*)s_lvl)[jn] + 1);
-                    }
-                    if (kb + 1 < m) {
-                        const int jn = (int)s_tmp[kb + 1];
-                        if (jn < i && (round * m + jn) % C == c) lv = max(lv, ((volatile int*)s_lvl)[jn] + 1);
-                    }
-                    if (lv != s_lvl[i]) { s_lvl[i] = lv; changed = 1; }
-                }
-                const bool again = __any_sync(0xffffffffu, changed);
-                __syncwarp();
-                if (!again) break;
-            }
-            int maxl = 0;
-            for (int i = lane; i < m; i += 32) maxl = max(maxl, s_lvl[i]);
-            const int L = __reduce_max_sync(0xffffffffu, maxl);
-            P.subtick(PROF_X_LEVELS);
-            for (int lv = 1; lv <= L; lv++) {
-                for (int i = lane; i < m; i += 32) {
-                    if (s_lvl[i] != lv) continue;
-                    const int kb = (int)s_order[i];
-                    const int a = round * m + i;
-                    const int c = a % C;
-                    const int k = c * nt + kb;
-                    const uint32_t r1 = B.slot[k], r2 = B.slot[k + 1];
-                    const double x = s_dbeta[kb] * (double)(B.E[r1] - B.E[r2]);
-                    s_att[k]++;
-                    if (x > 0.0 || (double)s_xlogu[a] < x) {
-                        s_succ[k]++;
-                        B.slot[k] = r2;
-                        B.slot[k + 1] = r1;
-                    }
-                }
-                __syncwarp();
-            }
-            P.subtick(PROF_X_APPLY);
-            // reshuffle: rank the pairs by fresh random keys (ties by position)
-            const uint32_t* keys = s_xrand + round * m;
-            for (int i = lane; i < m; i += 32) {
-                const uint32_t ki = keys[i];
-                int rank = 0;
-                for (int j = 0; j < m; j++) {
-                    const uint32_t kj = keys[j];
-                    rank += (kj < ki) || (kj == ki && j < i);
-                }
-                s_tmp[rank] = s_order[i];
-            }
-            __syncwarp();
-            for (int i = lane; i < m; i += 32) s_order[i] = s_tmp[i];
-            __syncwarp();
-            P.subtick(PROF_X_SHUFFLE);
+            s_next[kb] = rank;
         }
+        __syncwarp();
+        for (int kb = lane; kb < m; kb += 32) {
+            const int p = (int)s_pos[kb], c = (round * m + p) % C;
+            uint32_t w = (uint32_t)p | ((uint32_t)c << kPosBits);
+            if (kb > 0) {
+                const int q = (int)s_pos[kb - 1];
+                if (q < p && (round * m + q) % C == c) w |= kWaitLeft;
+            }
+            if (kb + 1 < m) {
+                const int q = (int)s_pos[kb + 1];
+                if (q < p && (round * m + q) % C == c) w |= kWaitRight;
+            }
+            keys[kb] = w;
+        }
+        __syncwarp();
+        for (int kb = lane; kb < m; kb += 32) s_pos[kb] = (uint32_t)s_next[kb];
+        __syncwarp();
+    }
+}
+
+__device__ void exchange_reference_order(const BlockCtx& B, const double* s_dbeta, unsigned* s_att, unsigned* s_succ,
+                                         const float* s_xlogu, const uint32_t* s_xrand, const uint32_t* s_pos,
+                                         uint32_t* s_order, int* s_done, const Prof P) {
+    const InstanceDesc& D = B.D;
+    const int nt = D.nt, C = D.chains, m = nt - 1;
+    if (m > 0 && threadIdx.x < 32) {
+        const int lane = threadIdx.x;
+        uint32_t* const slot = B.slot;
+        const long long* const E = B.E;
+        auto attempt = [&](int kb, uint32_t w, int round) {
+            const int k = (int)((w >> kPosBits) & 63u) * nt + kb;
+            const uint32_t r1 = slot[k], r2 = slot[k + 1];
+            s_att[k]++;
+            if (swap_accepted(s_dbeta[kb], E[r1] - E[r2], s_xlogu[round * m + (int)(w & ((1u << kPosBits) - 1u))])) {
+                s_succ[k]++;
+                slot[k] = r2;
+                slot[k + 1] = r1;
+            }
+        };
+        if (m <= 64) {
+            // two pairs per lane (lane, lane + 32), the attempts made as bits
+            // of one word: 20 pairs and two chains take 4.0 -> 2.2 us
+            for (int round = 0; round < C; round++) {
+                uint32_t w[2];
+                unsigned long long needs[2];   // attempts waited for
+#pragma unroll
+                for (int q = 0; q < 2; q++) {
+                    const int kb = lane + 32 * q;
+                    w[q] = kb < m ? s_xrand[round * m + kb] : 0u;
+                    needs[q] = (w[q] & kWaitLeft ? 1ull << ((kb - 1) & 63) : 0ull) |
+                               (w[q] & kWaitRight ? 1ull << ((kb + 1) & 63) : 0ull);
+                }
+                unsigned long long todo = m == 64 ? ~0ull : (1ull << m) - 1ull;
+                while (todo) {
+                    const bool g0 = ((todo >> lane) & 1ull) && !(needs[0] & todo);
+                    const bool g1 = ((todo >> (lane + 32)) & 1ull) && !(needs[1] & todo);
+                    if (g0) attempt(lane, w[0], round);
+                    if (g1) attempt(lane + 32, w[1], round);
+                    const unsigned long long made = (unsigned long long)__ballot_sync(0xffffffffu, g0) |
+                                                    ((unsigned long long)__ballot_sync(0xffffffffu, g1) << 32);
+                    if (made == 0) break;   // (cannot happen: the earliest attempt left waits for none)
+                    todo &= ~made;
+                    __syncwarp();
+                }
+            }
+        } else {
+            volatile int* const done = s_done;
+            for (int round = 0; round < C; round++) {
+                for (int kb = lane; kb < m; kb += 32) done[kb] = 0;
+                __syncwarp();
+                for (int left = m; left > 0;) {
+                    // the attempts that wait for none (marked 2 until all have looked)
+                    int made = 0;
+                    for (int kb = lane; kb < m; kb += 32) {
+                        const uint32_t w = s_xrand[round * m + kb];
+                        if (done[kb] == 0 && !((w & kWaitLeft) && done[kb - 1] != 1) && !((w & kWaitRight) && done[kb + 1] != 1)) {
+                            attempt(kb, w, round);
+                            done[kb] = 2;
+                            made++;
+                        }
+                    }
+                    __syncwarp();
+                    for (int kb = lane; kb < m; kb += 32)
+                        if (done[kb] == 2) done[kb] = 1;
+                    __syncwarp();
+                    made = __reduce_add_sync(0xffffffffu, made);
+                    if (made == 0) break;   // (as above)
+                    left -= made;
+                }
+            }
+        }
+        for (int kb = lane; kb < m; kb += 32) s_order[s_pos[kb]] = (uint32_t)kb;
+        P.subtick(PROF_X_APPLY);
     }
     __syncthreads();
-    (void)s_misc;
 }
 
 // Log-uniforms of the even/odd exchange: a thread's pair of each pass, drawn
@@ -1716,22 +1778,6 @@ __device__ __forceinline__ EvenOddDraws even_odd_draw(const EngineArgs& A, const
     if (tid < C * per0) u.lu0 = even_odd_log_u(A.seed, (uint32_t)D.inst_id, step, even_odd_pair(tid, 0, per0, nt, kb), 0);
     if (tid < C * per1) u.lu1 = even_odd_log_u(A.seed, (uint32_t)D.inst_id, step, even_odd_pair(tid, 1, per1, nt, kb), 1);
     return u;
-}
-
-// Accepts a swap with energy difference dE across dbeta: x = dbeta * dE > 0
-// or log u < x, in FP64.  The sign of x is the product of the signs, and the
-// comparison is decided in FP32 unless log u lies within 1e-5 of x relative
-// to |x| (the FP32 product is within 2^-21 of x), so that the FP64 pipe,
-// slow on this chip, is left to about one attempt in 10^5.
-__device__ __forceinline__ bool swap_accepted(double dbeta, long long dE, float log_u) {
-    const float db = (float)dbeta, xf = db * (float)dE;
-    if (dE == 0 && fabsf(db) < 1e30f) return log_u < 0.f;
-    if (fabsf(xf) > 1e-30f && fabsf(db) > 1e-30f) {
-        if (xf > 0.f) return true;
-        if (fabsf(log_u - xf) > 1e-5f * fabsf(xf)) return log_u < xf;
-    }
-    const double x = dbeta * (double)dE;
-    return x > 0.0 || (double)log_u < x;
 }
 
 // Deterministic even/odd exchange: per chain, all even pairs, then all odd
@@ -2022,6 +2068,14 @@ __global__ void __launch_bounds__((REPLAY || (BLOCKTEAM && !NARROW)) ? 1024 : kN
         // the exchange's draws, before the wait for the energies
         EvenOddDraws xdraw{0.f, 0.f};
         const bool even_odd = !REPLAY && (A.phase_mask & PHASE_EXCHANGE) && (A.flags & ENGINE_EXCHANGE_EVEN_ODD);
+        const bool ordered = !REPLAY && (A.phase_mask & PHASE_EXCHANGE) && !(A.flags & ENGINE_EXCHANGE_EVEN_ODD) && nt > 1;
+        auto draw = [&]() {
+            if (even_odd) xdraw = even_odd_draw(A, D, step);
+            if (ordered) {
+                exchange_reference_draw(A, D, step, s_xlogu, s_xrand);
+                if (tid < 32) exchange_reference_plan(D, s_order, s_xrand, s_tmp, s_lvl);
+            }
+        };
         // Publishes this block's spins (for ICM partners) as words of 32
         // sites carrying the step's tag: a partner checks the tag of each
         // word it reads, so nothing orders these stores and no fence waits
@@ -2068,7 +2122,7 @@ __global__ void __launch_bounds__((REPLAY || (BLOCKTEAM && !NARROW)) ? 1024 : kN
                 else st_relaxed_gpu_u64(ew + (B.r0 + j) * kPubStride, w);
             }
             if (icm_on) publish_spins();
-            if (even_odd) xdraw = even_odd_draw(A, D, step);
+            draw();
             const unsigned long long limit = A.wait_limit_ns ? A.wait_limit_ns : kWaitLimitNs;
             int ok = 1;
             bool polled = false;
@@ -2097,15 +2151,15 @@ __global__ void __launch_bounds__((REPLAY || (BLOCKTEAM && !NARROW)) ? 1024 : kN
             // publish this block's energies (and spins, for ICM partners)
             for (int j = tid; j < rpc; j += T) A.energy_pub[parity * A.energy_pub_half + D.rep_off + B.r0 + j] = B.E[B.r0 + j];
             if (icm_on) publish_spins();
-            if (even_odd) xdraw = even_odd_draw(A, D, step);
+            draw();
             if (!group_barrier(A.bar + 2 * inst, (unsigned)(D.group + A.bar_phantom), abortf, A.status, bar_gen,
                                A.wait_limit_ns ? A.wait_limit_ns : kWaitLimitNs))
                 break;
             for (int r = tid; r < R; r += T)
                 if (r < B.r0 || r >= B.r0 + rpc) B.E[r] = ld_cg(A.energy_pub + parity * A.energy_pub_half + D.rep_off + r);
             __syncthreads();
-        } else if (even_odd) {
-            xdraw = even_odd_draw(A, D, step);
+        } else {
+            draw();
         }
         P.tick(PROF_BARRIER);
         if (A.hist != nullptr && D.hist_nbins > 0 && step >= A.hist_from && B.rank == 0) {
@@ -2128,7 +2182,7 @@ __global__ void __launch_bounds__((REPLAY || (BLOCKTEAM && !NARROW)) ? 1024 : kN
         if (A.phase_mask & PHASE_EXCHANGE) {
             if (REPLAY) exchange_replay(A, B, ls, s_beta, s_att, s_succ);
             else if (A.flags & ENGINE_EXCHANGE_EVEN_ODD) exchange_even_odd(A, B, step, s_dbeta, s_att, s_succ, xdraw);
-            else exchange_reference_order(A, B, step, s_order, s_dbeta, s_att, s_succ, s_xlogu, s_xrand, s_lvl, s_tmp, s_misc, P);
+            else exchange_reference_order(B, s_dbeta, s_att, s_succ, s_xlogu, s_xrand, s_tmp, s_order, s_lvl, P);
             for (int s = tid; s < R; s += T) {
                 const uint32_t r = B.slot[s];
                 if ((int)r >= B.r0 && (int)r < B.r0 + rpc) {
