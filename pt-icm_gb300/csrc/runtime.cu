@@ -34,6 +34,12 @@ cudaError_t launch_init_spins(const EngineArgs& A, const int32_t* rep_inst, int 
 cudaError_t launch_evaluate(const int32_t* row, const uint32_t* adj, const int32_t* h, int n, int n_pad,
                             const int8_t* states, int count, long long* E_out, long long* cut2_out,
                             int32_t* dE_out, cudaStream_t stream);
+cudaError_t launch_export(const int8_t* spins, const int32_t* fields, const int32_t* iperm, uint8_t* states_out,
+                          int32_t* fields_out, int R, int n, int n_pad, cudaStream_t stream);
+size_t evaluate_states_smem(int n, bool with_dE);
+cudaError_t launch_evaluate_states(const int32_t* row, const uint32_t* adj, const int32_t* h, const int32_t* iperm, int n,
+                                   const uint8_t* states, int count, long long* E_out, long long* cut2_out,
+                                   double* dE_out, cudaStream_t stream);
 cudaError_t launch_philox_probe(const uint4* ctr, const uint2* key, uint4* out, int count, cudaStream_t stream);
 }  // namespace pticm
 
@@ -104,7 +110,8 @@ struct pticm_ctx {
     DArr<unsigned int> d_bar;
     DArr<int> d_abort;
     DArr<DevStatus> d_status;
-    DArr<uint8_t> d_states_in;  // caller states in the original site order (pticm_set_states)
+    DArr<uint8_t> d_states_in;  // states in the original site order (pticm_set_states, pticm_get_replicas)
+    DArr<int32_t> d_fields_out; // fields in the original site order (pticm_get_replicas)
     DArr<uint8_t> d_icm_pool;   // ICM scratch when the replicas live in device memory
     long long icm_stride = 0;
     long long ebound = -1;      // energy_bound(P), once
@@ -945,6 +952,32 @@ int pticm_problem_evaluate(const pticm_problem* pc, int64_t count, const uint8_t
     const int n = (int)P.n, npad = pad16(n);
     ProblemDevice PD;
     if (int rc = problem_device(p, &PD)) return rc;
+    if (evaluate_states_smem(n, dE != nullptr) <= kSmemLimit) {
+        // in portions of at most 64 MB of results
+        const int64_t per = std::max<int64_t>(1, std::min<int64_t>(count, (64ll << 20) / ((int64_t)n * (dE ? 8 : 1))));
+        DArr<uint8_t> d_in;
+        DArr<long long> d_E, d_c;
+        DArr<double> d_dE;
+        CK(d_in.reserve((size_t)per * n));
+        CK(d_E.reserve(per));
+        CK(d_c.reserve(per));
+        if (dE) CK(d_dE.reserve((size_t)per * n));
+        std::vector<long long> E(per), C2(per);
+        for (int64_t g0 = 0; g0 < count; g0 += per) {
+            const int64_t cnt = std::min(per, count - g0);
+            CK(cudaMemcpy(d_in.p, states + g0 * n, (size_t)cnt * n, cudaMemcpyHostToDevice));
+            CK(launch_evaluate_states(PD.row, PD.adj, P.has_h ? PD.h : nullptr, PD.iperm, n, d_in.p, (int)cnt, d_E.p, d_c.p,
+                                      dE ? d_dE.p : nullptr, nullptr));
+            CK(cudaMemcpy(E.data(), d_E.p, (size_t)cnt * 8, cudaMemcpyDeviceToHost));
+            CK(cudaMemcpy(C2.data(), d_c.p, (size_t)cnt * 8, cudaMemcpyDeviceToHost));
+            if (dE) CK(cudaMemcpy(dE + g0 * n, d_dE.p, (size_t)cnt * n * 8, cudaMemcpyDeviceToHost));
+            for (int64_t g = 0; g < cnt; g++) {
+                if (energy) energy[g0 + g] = (double)E[g];
+                if (maxcut) maxcut[g0 + g] = 0.5 * (double)C2[g];
+            }
+        }
+        return PTICM_OK;
+    }
     std::vector<int8_t> dev((size_t)count * npad, 1);
     for (int64_t g = 0; g < count; g++)
         for (int i = 0; i < n; i++) dev[g * npad + i] = states[g * n + P.perm[i]] ? 1 : -1;
@@ -1299,17 +1332,17 @@ int pticm_get_replicas(pticm_ctx* c, uint8_t* states, int64_t* energy, int32_t* 
     if (!c) return fail(PTICM_ERR_INVALID, "null argument");
     CK(cudaStreamSynchronize(c->stream));
     const int n = (int)c->P.n, npad = c->desc.n_pad;
-    if (states) {
-        std::vector<int8_t> s;
-        CK(c->d_spins.download(s));
-        for (int r = 0; r < c->R; r++)
-            for (int i = 0; i < n; i++) states[(size_t)r * n + c->P.perm[i]] = s[(size_t)r * npad + i] > 0 ? 1 : 0;
-    }
-    if (fields) {
-        std::vector<int32_t> f;
-        CK(c->d_fields.download(f));
-        for (int r = 0; r < c->R; r++)
-            for (int i = 0; i < n; i++) fields[(size_t)r * n + c->P.perm[i]] = f[(size_t)r * npad + i];
+    if (states || fields) {
+        // into the original order on the device, then straight to the caller
+        const size_t sites = (size_t)c->R * (size_t)n;
+        DArr<int32_t>& d_f = c->d_fields_out;
+        if (states && c->d_states_in.n != sites) CK(c->d_states_in.reserve(sites));
+        if (fields && d_f.n != sites) CK(d_f.reserve(sites));
+        CK(launch_export(c->d_spins.p, c->d_fields.p, c->d_perm.p, states ? c->d_states_in.p : nullptr, fields ? d_f.p : nullptr, c->R, n, npad,
+                         c->stream));
+        if (states) CK(cudaMemcpyAsync(states, c->d_states_in.p, sites, cudaMemcpyDeviceToHost, c->stream));
+        if (fields) CK(cudaMemcpyAsync(fields, d_f.p, sites * sizeof(int32_t), cudaMemcpyDeviceToHost, c->stream));
+        CK(cudaStreamSynchronize(c->stream));
     }
     if (energy) {
         std::vector<long long> e;

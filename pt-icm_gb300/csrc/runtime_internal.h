@@ -28,13 +28,18 @@ struct DArr {
         p = nullptr;
         n = 0;
     }
-    cudaError_t alloc(size_t count) {
+    // uninitialised, for buffers that a kernel or copy fills
+    cudaError_t reserve(size_t count) {
         release();
         n = count;
         if (count == 0) return cudaSuccess;
-        cudaError_t e = cudaMalloc(&p, count * sizeof(T));
-        if (e != cudaSuccess) { p = nullptr; n = 0; return e; }
-        return cudaMemset(p, 0, count * sizeof(T));
+        const cudaError_t e = cudaMalloc(&p, count * sizeof(T));
+        if (e != cudaSuccess) { p = nullptr; n = 0; }
+        return e;
+    }
+    cudaError_t alloc(size_t count) {
+        const cudaError_t e = reserve(count);
+        return e != cudaSuccess || count == 0 ? e : cudaMemset(p, 0, count * sizeof(T));
     }
     cudaError_t upload(const std::vector<T>& v, size_t extra = 0) {
         cudaError_t e = alloc(v.size() + extra);
