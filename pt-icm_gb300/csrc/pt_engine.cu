@@ -190,6 +190,16 @@ enum Space : int {
     SP_SHARED = 1,   // adjacency staged; replicas, thresholds and cluster scratch in shared memory
     SP_STATE = 2,    // as SP_SHARED, but the adjacency may be in device memory (an instance of a batch)
     SP_LARGE = 3,    // spins and cluster scratch in shared memory; adjacency, thresholds and the overlap list in device memory
+    SP_LARGE4 = 4,   // as SP_LARGE with four replicas in the block, their spins interleaved: byte 4 i + j is replica j's site i
+};
+constexpr bool space_large(int space) { return space == SP_LARGE || space == SP_LARGE4; }
+constexpr int space_stride(int space) { return space == SP_LARGE4 ? 4 : 1; }   // bytes between a replica's sites
+
+// One replica's spins in a block.
+template <int SPACE>
+struct SpinRow {
+    int8_t* p;
+    __device__ __forceinline__ int8_t& operator[](int i) const { return p[space_stride(SPACE) * i]; }
 };
 
 // The cluster search unites along every edge, instead of sampling links first,
@@ -217,6 +227,11 @@ struct BlockCtx {
     uint32_t* rslot;
     int32_t* tb;        // threshold row base of each local replica
 };
+
+template <int SPACE>
+__device__ __forceinline__ SpinRow<SPACE> spin_row(const BlockCtx& B, int j) {
+    return SpinRow<SPACE>{B.spin + (SPACE == SP_LARGE4 ? j : j * B.D.n_pad)};
+}
 
 // ICM team scratch: BFS queue / union-find parents (n ints), overlap flags
 // (n bytes), visited bits (icm_team_bytes); a block team's overlap list (n
@@ -310,8 +325,7 @@ __device__ __forceinline__ int icm_pair(const EngineArgs& A, const BlockCtx& B, 
     auto pub_site = [&](const unsigned long long* pub, int i) -> int8_t {
         return ((pub_bits(ld_relaxed_gpu_u64(pub + (i >> 5))) >> (i & 31)) & 1u) ? (int8_t)1 : (int8_t)-1;
     };
-    int8_t* sA = locA ? B.spin + (rA - B.r0) * npad : nullptr;
-    int8_t* sB = locB ? B.spin + (rB - B.r0) * npad : nullptr;
+    const SpinRow<SPACE> sA = spin_row<SPACE>(B, locA ? rA - B.r0 : 0), sB = spin_row<SPACE>(B, locB ? rB - B.r0 : 0);
     // no stored fields in field_gather mode: field updates are skipped
     int32_t* fA = (locA && B.field) ? B.field + (rA - B.r0) * npad : nullptr;
     int32_t* fB = (locB && B.field) ? B.field + (rB - B.r0) * npad : nullptr;
@@ -386,8 +400,19 @@ __device__ __forceinline__ int icm_pair(const EngineArgs& A, const BlockCtx& B, 
         // the next round's words are loaded before this round's are used
         // (a partner's words come from L2)
         auto load_words = [&](int w, unsigned long long& wa, unsigned long long& wb) {
-            wa = locA ? reinterpret_cast<const uint32_t*>(sA)[w] : ld_relaxed_gpu_u64(pubA + (w >> 3));
-            wb = locB ? reinterpret_cast<const uint32_t*>(sB)[w] : ld_relaxed_gpu_u64(pubB + (w >> 3));
+            if (SPACE == SP_LARGE4) {
+                // byte j of four words, put together
+                const uint4 q = reinterpret_cast<const uint4*>(B.spin)[w];
+                auto quad = [&](int j) -> uint32_t {
+                    const uint32_t sel = (uint32_t)j | ((uint32_t)(4 + j) << 4);
+                    return __byte_perm(__byte_perm(q.x, q.y, sel), __byte_perm(q.z, q.w, sel), 0x5410);
+                };
+                wa = locA ? quad(rA - B.r0) : ld_relaxed_gpu_u64(pubA + (w >> 3));
+                wb = locB ? quad(rB - B.r0) : ld_relaxed_gpu_u64(pubB + (w >> 3));
+            } else {
+                wa = locA ? reinterpret_cast<const uint32_t*>(sA.p)[w] : ld_relaxed_gpu_u64(pubA + (w >> 3));
+                wb = locB ? reinterpret_cast<const uint32_t*>(sB.p)[w] : ld_relaxed_gpu_u64(pubB + (w >> 3));
+            }
         };
         unsigned long long na = 0, nb = 0;
         if (team.tr < nq) load_words(team.tr, na, nb);
@@ -703,7 +728,7 @@ __device__ __forceinline__ int icm_pair(const EngineArgs& A, const BlockCtx& B, 
                 // (GLINK: with the neighbour lists in device memory, a
                 // thread scans four of its sites side by side, so that
                 // their dependent loads overlap)
-                const bool glink = GLINK && BLOCK && (SPACE == SP_LARGE || !__isShared(badj)) &&
+                const bool glink = GLINK && BLOCK && (space_large(SPACE) || !__isShared(badj)) &&
                                    (reinterpret_cast<uintptr_t>(badj) & 15u) == 0;
                 // (a block team's round 0 keeps the link left for round 1, by
                 // list position, in the free part of the list: S is listed
@@ -1153,7 +1178,8 @@ __device__ __forceinline__ int icm_pair(const EngineArgs& A, const BlockCtx& B, 
 
 // Local field of site i gathered from the neighbours' spins (field_gather
 // mode, where fields are not stored): f_i = sum_j J_ij s_j.
-__device__ __forceinline__ int gather_field(const int32_t* row, const uint32_t* adj, const int8_t* sp, int i) {
+template <class Spins>
+__device__ __forceinline__ int gather_field(const int32_t* row, const uint32_t* adj, Spins sp, int i) {
     int f = 0;
     for_each_neighbour(row, adj, i, [&](uint32_t e) { f += (int)(int8_t)(e & 0xffu) * sp[e >> 8]; });
     return f;
@@ -1188,6 +1214,87 @@ __device__ __forceinline__ int gather_pieces(const int32_t* row, const uint32_t*
     return f;
 }
 
+// The local fields of four interleaved replicas at one site per lane (its list
+// of my_deg entries from my0; 0 entries: none).  Four neighbouring lanes gather one another's sites in turn, each
+// a quarter of the list's 16-byte pieces, so that a group's loads are whole
+// sectors of one list; one 32-bit load brings a neighbour's spin in all four
+// replicas.  What bounds it is that load's bank conflicts and the lists' way
+// from L2: 215 us a sweep of N=20000, degree 40, 4 replicas on each of 128
+// SMs.  (One thread per site and a byte load per replica, four times the
+// shared wavefronts and an L1 lookup per lane and piece: 413 us; without the
+// pieces loaded ahead: 267 us.)
+// PACKED (no field beyond +-127): with the four spins as signed digits of a
+// 32-bit number, base 256, one multiply-add sums all four fields, modulo 2^32;
+// the digits are taken apart at the end.
+// The first kAhead pieces of all four sites are loaded before the first is
+// used: a warp waits for L2 once per 32 sites.
+template <bool PACKED>
+__device__ __forceinline__ void gather4(const uint32_t* adj, const uint32_t* s4, int my0, int my_deg, int (&f)[4]) {
+    constexpr int kAhead = 3;
+    const int lane = threadIdx.x & 31, sub = lane & 3;
+    const uint4* const adj4 = reinterpret_cast<const uint4*>(adj);
+    uint4 ahead[4][kAhead];
+#pragma unroll
+    for (int s = 0; s < 4; s++) {
+        const int src = (lane & ~3) + s;
+        const int e0 = __shfl_sync(0xffffffffu, my0, src), deg = __shfl_sync(0xffffffffu, my_deg, src);
+        const int p0 = (e0 >> 2) + sub, p1 = (e0 + deg + 3) >> 2;
+#pragma unroll
+        for (int x = 0; x < kAhead; x++)
+            ahead[s][x] = p0 + 4 * x < p1 ? adj4[p0 + 4 * x] : make_uint4(0, 0, 0, 0);
+    }
+#pragma unroll
+    for (int s = 0; s < 4; s++) {
+        const int src = (lane & ~3) + s;
+        const int e0 = __shfl_sync(0xffffffffu, my0, src), deg = __shfl_sync(0xffffffffu, my_deg, src);
+        const int p0 = (e0 >> 2) + sub, p1 = (e0 + deg + 3) >> 2;
+        int acc = 0, g[4] = {0, 0, 0, 0};
+        auto piece = [&](const uint4& q, int p) {
+            uint32_t e[4] = {q.x, q.y, q.z, q.w}, r[4];
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                if ((unsigned)(4 * p + k - e0) >= (unsigned)deg) e[k] = 0;
+                r[k] = s4[e[k] >> 8];
+            }
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                const int w = (int)(int8_t)(e[k] & 0xffu);
+                if (PACKED) {
+                    // bytes to digits: a negative digit borrows from the next
+                    acc += w * (int)(r[k] - ((r[k] & 0x00808080u) << 1));
+                } else {
+#pragma unroll
+                    for (int j = 0; j < 4; j++) g[j] += w * (int)(int8_t)(r[k] >> (8 * j));
+                }
+            }
+        };
+#pragma unroll
+        for (int x = 0; x < kAhead; x++) piece(ahead[s][x], p0 + 4 * x);
+#pragma unroll 1
+        for (int p = p0 + 4 * kAhead; p < p1; p += 4) piece(adj4[p], p);
+        if (PACKED) {
+            acc += __shfl_xor_sync(0xffffffffu, acc, 1);
+            acc += __shfl_xor_sync(0xffffffffu, acc, 2);
+            if (sub == s) f[0] = acc;
+        } else {
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                g[j] += __shfl_xor_sync(0xffffffffu, g[j], 1);
+                g[j] += __shfl_xor_sync(0xffffffffu, g[j], 2);
+                if (sub == s) f[j] = g[j];
+            }
+        }
+    }
+    if (PACKED) {
+        int acc = f[0];
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            f[j] = (int)(int8_t)(acc & 0xff);
+            acc = (acc - f[j]) >> 8;
+        }
+    }
+}
+
 // --------------------------------------------------------------- sweeps
 // A warp pushes the field changes of at most this many accepted sites one
 // site at a time (a lane per neighbour); with more, each lane pushes its own
@@ -1207,7 +1314,7 @@ constexpr int kGatherReps = 4;
 // a phase boundary; with several, warps aggregate per replica before touching
 // shared memory.  COOP: the narrow block team, whose instances with few
 // neighbours gather (InstanceDesc::lanes), and whose others push together.
-template <bool ONE, bool COOP>
+template <bool ONE, bool COOP, int SPACE>
 __device__ void colored_sweep(const EngineArgs& A, const BlockCtx& B, unsigned long long sweep_idx,
                               int32_t* s_col, const uint32_t* s_thr, int* s_dEp, unsigned* s_flp,
                               unsigned long long* s_flips, long long* s_bestE, int* s_improved,
@@ -1343,6 +1450,60 @@ __device__ void colored_sweep(const EngineArgs& A, const BlockCtx& B, unsigned l
                         for_each_neighbour(row, adj, i,
                                            [&](uint32_t e) { atomicAdd(fd + (e >> 8), (int)(int8_t)(e & 0xffu) * dl); });
                     }
+                }
+            }
+        } else if (SPACE == SP_LARGE4) {
+            // (the four replicas' energy changes and flips: one addition per
+            // warp, replica and class)
+            int g_de[4] = {0, 0, 0, 0};
+            unsigned g_fl[4] = {0, 0, 0, 0};
+            uint32_t* const s4 = reinterpret_cast<uint32_t*>(B.spin);
+            int e0 = 0, deg = 0;   // (of the site after this one)
+            auto list_of = [&](int i) {
+                e0 = 0;
+                deg = 0;
+                if (i < c0 + Sc) {
+                    e0 = row[i];
+                    deg = row[i + 1] - e0;
+                }
+            };
+            list_of(c0 + tid);
+            for (int base = c0 + (tid & ~31); base < c0 + Sc; base += T) {
+                const int i = base + lane;
+                int f[4];
+                const int a0 = e0, ad = deg;
+                list_of(i + T);
+                if (kmax <= 127) gather4<true>(adj, s4, a0, ad, f);
+                else gather4<false>(adj, s4, a0, ad, f);
+                if (i >= c0 + Sc) continue;
+                const int hi = B.h ? B.h[i] : 0;
+                uint32_t w = s4[i];
+                const uint32_t w0 = w;
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    const int s = (int)(int8_t)(w0 >> (8 * j));
+                    const int de = -2 * s * (f[j] + hi);
+                    bool acc = de <= 0;
+                    if (!acc) {
+                        const uint32_t thr = s_thr[B.tb[j] + min(de >> 1, kmax)];
+                        acc = (rng.next() < thr) || (thr == 0xFFFFFFFFu);
+                    }
+                    if (acc) {
+                        w ^= 0xFEu << (8 * j);   // 0x01 <-> 0xFF
+                        g_de[j] += de;
+                        g_fl[j]++;
+                    }
+                }
+                if (w != w0) s4[i] = w;
+            }
+            __syncwarp();
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                const int v = (int)__reduce_add_sync(0xffffffffu, (unsigned)g_de[j]);
+                const unsigned f = __reduce_add_sync(0xffffffffu, g_fl[j]);
+                if (lane == 0 && f != 0) {
+                    atomicAdd(s_dEp + j, v);
+                    atomicAdd(s_flp + j, f);
                 }
             }
         } else if (gm) {
@@ -1498,7 +1659,8 @@ __device__ void colored_sweep(const EngineArgs& A, const BlockCtx& B, unsigned l
         if (s_misc[1] > 0) {
             for (int idx = tid; idx < rpc * npad; idx += T) {
                 const int j = ONE ? 0 : idx / npad;
-                if (s_improved[j]) A.best_state[D.spin_off + (long long)B.r0 * npad + idx] = B.spin[idx];
+                if (s_improved[j])
+                    A.best_state[D.spin_off + (long long)B.r0 * npad + idx] = spin_row<SPACE>(B, j)[idx - j * npad];
             }
             __syncthreads();
             if (tid == 0) s_misc[1] = 0;
@@ -1884,7 +2046,7 @@ __global__ void __launch_bounds__((REPLAY || (BLOCKTEAM && !NARROW)) ? 1024 : kN
     int32_t* s_h = sm_ptr<int32_t>(smem, S.h);
     // acceptance thresholds: shared memory, or read through L1 (field_gather)
     uint32_t* s_thr_w = sm_ptr<uint32_t>(smem, S.thr);
-    const bool thr_global = SPACE == SP_LARGE || (SPACE == SP_ANY && S.field_gather);
+    const bool thr_global = space_large(SPACE) || (SPACE == SP_ANY && S.field_gather);
     const uint32_t* s_thr = thr_global ? A.thr + D.thr_off : s_thr_w;
     double* s_ptab = sm_ptr<double>(smem, S.ptab);
     uint32_t* s_order = sm_ptr<uint32_t>(smem, S.order);
@@ -1945,7 +2107,7 @@ __global__ void __launch_bounds__((REPLAY || (BLOCKTEAM && !NARROW)) ? 1024 : kN
     BlockCtx B{D, rank, rep0};
     B.spin = sm_ptr<int8_t>(smem, S.spin);
     // (a narrow block team with lanes gathers its fields)
-    B.field = (BLOCKTEAM && NARROW && D.lanes > 0) || SPACE == SP_LARGE || (SPACE == SP_ANY && S.field_gather) ? nullptr : sm_ptr<int32_t>(smem, S.field);
+    B.field = (BLOCKTEAM && NARROW && D.lanes > 0) || space_large(SPACE) || (SPACE == SP_ANY && S.field_gather) ? nullptr : sm_ptr<int32_t>(smem, S.field);
     if (SPACE == SP_ANY && S.state_global) {
         // replicas too large for shared memory work on their master copy
         B.spin = A.spins + D.spin_off + (long long)rep0 * D.n_pad;
@@ -1958,7 +2120,7 @@ __global__ void __launch_bounds__((REPLAY || (BLOCKTEAM && !NARROW)) ? 1024 : kN
     B.h = D.has_h ? s_h : nullptr;
     B.row = sm_ptr<int32_t>(smem, S.row);
     B.adj = sm_ptr<uint32_t>(smem, S.adj);
-    if (SPACE == SP_LARGE || (SPACE != SP_SHARED && !staged)) {
+    if (space_large(SPACE) || (SPACE != SP_SHARED && !staged)) {
         B.row = g_row;
         B.adj = g_adj;
     }
@@ -1968,7 +2130,8 @@ __global__ void __launch_bounds__((REPLAY || (BLOCKTEAM && !NARROW)) ? 1024 : kN
     if (!S.state_global) {
         const long long base = D.spin_off + (long long)B.r0 * npad;
         for (int idx = tid; idx < rpc * npad; idx += T) {
-            B.spin[idx] = A.spins[base + idx];
+            const int j = space_stride(SPACE) == 1 ? 0 : idx / npad;
+            spin_row<SPACE>(B, j)[idx - j * npad] = A.spins[base + idx];
             if (B.field) B.field[idx] = A.fields[base + idx];
         }
     }
@@ -2043,7 +2206,7 @@ __global__ void __launch_bounds__((REPLAY || (BLOCKTEAM && !NARROW)) ? 1024 : kN
                     replay_sweep(A, B, ls, sw, sweep_idx, s_ptab, s_flips, s_bestE);
                     __syncthreads();
                 } else {
-                    colored_sweep<BLOCKTEAM, BLOCKTEAM && NARROW>(A, B, sweep_idx, s_col, s_thr, s_dEp, s_flp, s_flips, s_bestE,
+                    colored_sweep<BLOCKTEAM, BLOCKTEAM && NARROW, SPACE>(A, B, sweep_idx, s_col, s_thr, s_dEp, s_flp, s_flips, s_bestE,
                                              s_improved, s_misc, best_pp);
                 }
             }
@@ -2056,7 +2219,7 @@ __global__ void __launch_bounds__((REPLAY || (BLOCKTEAM && !NARROW)) ? 1024 : kN
             const int warp = tid >> 5, lane = tid & 31;
             for (int j = warp; j < rpc; j += (T >> 5)) {
                 long long m = 0;
-                for (int i = lane; i < n; i += 32) m += B.spin[(long long)j * npad + i];
+                for (int i = lane; i < n; i += 32) m += spin_row<SPACE>(B, j)[i];
                 for (int o = 16; o > 0; o >>= 1) m += __shfl_xor_sync(0xffffffffu, m, o);
                 if (lane == 0) s_mag[j] = m;
             }
@@ -2087,7 +2250,26 @@ __global__ void __launch_bounds__((REPLAY || (BLOCKTEAM && !NARROW)) ? 1024 : kN
             const unsigned long long tagw = (unsigned long long)(A.pub_base + (uint32_t)ls) << 32;
             unsigned long long* const out = A.spins_pub + parity * A.spins_pub_half + (D.spin_off >> 4) + (long long)B.r0 * npw;
             const int8_t* const sp = B.spin;
-            for (int j = 0; j < rpc; j++)
+            if (SPACE == SP_LARGE4) {
+                // (32 interleaved words give a word of each replica)
+                for (int k = tid; k < W; k += T) {
+                    uint32_t bits[4] = {0, 0, 0, 0};
+                    const uint4* const q = reinterpret_cast<const uint4*>(sp + 128 * (long long)k);
+#pragma unroll
+                    for (int x4 = 0; x4 < 8; x4++) {
+                        if (32 * k + 4 * x4 >= npad) break;
+                        const uint4 v = q[x4];
+                        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+                        for (int x = 0; x < 4; x++)
+#pragma unroll
+                            for (int j = 0; j < 4; j++) bits[j] |= ((~w[x] >> (8 * j + 7)) & 1u) << (4 * x4 + x);
+                    }
+#pragma unroll
+                    for (int j = 0; j < 4; j++) st_relaxed_gpu_u64(out + (long long)j * npw + k, tagw | bits[j]);
+                }
+            }
+            for (int j = 0; space_stride(SPACE) == 1 && j < rpc; j++)
                 for (int k = tid; k < W; k += T) {
                     const uint4* const q = reinterpret_cast<const uint4*>(sp + (long long)j * npad + 32 * k);
                     uint32_t v[8] = {};
@@ -2206,7 +2388,7 @@ __global__ void __launch_bounds__((REPLAY || (BLOCKTEAM && !NARROW)) ? 1024 : kN
             if (BLOCKTEAM || D.teams == 1) {
                 const Team<true> team{tid, T, s_team_ctl, s_team_keys};
                 IcmScratch X = icm_scratch(s_icm, npad);
-                if (SPACE == SP_LARGE || (SPACE == SP_ANY && !BLOCKTEAM && !REPLAY && S.icm_split))
+                if (space_large(SPACE) || (SPACE == SP_ANY && !BLOCKTEAM && !REPLAY && S.icm_split))
                     X.list = reinterpret_cast<int*>(g_icm);
                 for (int j = 0; j < rpc; j++) {
                     const int sl = (int)B.rslot[j], c = sl / nt, k = sl - c * nt, kk = nt - 1 - k;
@@ -2250,14 +2432,15 @@ __global__ void __launch_bounds__((REPLAY || (BLOCKTEAM && !NARROW)) ? 1024 : kN
     const long long base = D.spin_off + (long long)B.r0 * npad;
     if (SPACE != SP_ANY || !S.state_global)
         for (int idx = tid; idx < rpc * npad; idx += T) {
-            A.spins[base + idx] = B.spin[idx];
+            const int j = space_stride(SPACE) == 1 ? 0 : idx / npad;
+            A.spins[base + idx] = spin_row<SPACE>(B, j)[idx - j * npad];
             if (B.field) A.fields[base + idx] = B.field[idx];
         }
     if (!B.field) {
         // the stored fields of the master copy, gathered once per launch
         for (int idx = tid; idx < rpc * npad; idx += T) {
             const int j = idx / npad, i = idx - j * npad;
-            A.fields[base + idx] = i < n ? gather_field(B.row, B.adj, B.spin + (long long)j * npad, i) : 0;
+            A.fields[base + idx] = i < n ? gather_field(B.row, B.adj, spin_row<SPACE>(B, j), i) : 0;
         }
     }
     for (int j = tid; j < rpc; j += T) {
@@ -2488,6 +2671,7 @@ static void* engine_fn(bool replay, bool block_team, bool narrow, int space) {
     if (block_team) return (void*)pt_engine_kernel<false, true, false, SP_ANY>;
     if (space == SP_SHARED || space == SP_STATE) return (void*)pt_engine_kernel<false, false, false, SP_STATE>;
     if (space == SP_LARGE) return (void*)pt_engine_kernel<false, false, false, SP_LARGE>;
+    if (space == SP_LARGE4) return (void*)pt_engine_kernel<false, false, false, SP_LARGE4>;
     return (void*)pt_engine_kernel<false, false, false, SP_ANY>;
 }
 
@@ -2495,7 +2679,7 @@ static void* engine_fn(bool replay, bool block_team, bool narrow, int space) {
 // stages that instance; a batch stages some of its instances.)
 static int plan_space(const SmemPlan& S, bool block_team) {
     if (!S.state_global && !S.field_gather) return S.stage_adj && block_team ? SP_SHARED : SP_STATE;
-    if (S.field_gather && S.icm_split) return SP_LARGE;
+    if (S.field_gather && S.icm_split) return S.rpc == 4 ? SP_LARGE4 : SP_LARGE;
     return SP_ANY;
 }
 
@@ -2526,7 +2710,7 @@ cudaError_t engine_max_blocks_per_sm(bool replay, bool block_team, bool narrow, 
     }
     // the launch takes one of the variants by its plan: what all of them hold
     *out = 1 << 20;
-    for (int space : {SP_ANY, SP_SHARED, SP_STATE, SP_LARGE}) {
+    for (int space : {SP_ANY, SP_SHARED, SP_STATE, SP_LARGE, SP_LARGE4}) {
         const void* fn = engine_fn(replay, block_team, narrow, space);
         cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         int per_sm = 0;

@@ -209,6 +209,7 @@ SmemPlan layout_plan(const PlanDims& d) {
     S.max_kmax = (int32_t)d.max_kmax;
     S.max_R = (int32_t)d.R;
     S.max_nt = (int32_t)d.nt;
+    S.rpc = (int32_t)d.rpc;
     return S;
 }
 
