@@ -291,19 +291,23 @@ __device__ __forceinline__ void for_each_neighbour(const int32_t* row, const uin
 // change by -2 s_u h_u per flipped site plus -2 J s_u s_v per edge leaving
 // the set (s_v equal in A and B), an exact integer update.  Members held by
 // another block are read from the published copy and flipped by their own
-// block, which finds the same set.
+// block, which finds the same set -- or, given `result`, the block only writes
+// what is to be flipped (apply_pairs).
 template <bool BLOCK, bool REPLAY, bool LS, int SPACE, bool GLINK = false>
 __device__ __forceinline__ int icm_pair(const EngineArgs& A, const BlockCtx& B, const Team<BLOCK>& team, int q,
                                         int rA, int rB, unsigned long long step, int ls, const IcmScratch& X,
-                                        int where_err, const Prof P) {
+                                        int where_err, const Prof P, unsigned long long* result = nullptr) {
     const InstanceDesc& D = B.D;
     const int n = D.n, npad = D.n_pad;
     const int32_t* const brow = B.row;
     const uint32_t* const badj = B.adj;
     const int32_t* const bh = B.h;
     const bool has_h = bh != nullptr;
-    const bool locA = rA >= B.r0 && rA < B.r0 + D.rpc;
-    const bool locB = rB >= B.r0 && rB < B.r0 + D.rpc;
+    // (share: the result goes to the blocks that hold the replicas, and the
+    // published words serve as both states)
+    const bool share = space_large(SPACE) && result != nullptr;
+    const bool locA = !share && rA >= B.r0 && rA < B.r0 + D.rpc;
+    const bool locB = !share && rB >= B.r0 && rB < B.r0 + D.rpc;
     const int parity = (int)(step & 1ull);
     // a member held by another block: its published words of this step
     const unsigned long long* const pub0 = A.spins_pub + parity * A.spins_pub_half + (D.spin_off >> 4);
@@ -490,7 +494,7 @@ __device__ __forceinline__ int icm_pair(const EngineArgs& A, const BlockCtx& B, 
             }
         }
     }
-    if (algo == ENGINE_ICM_BFS)   // the visited bits of the breadth-first search
+    if (algo == ENGINE_ICM_BFS || share)   // the visited bits of the breadth-first search; the flipped set's
         for (int w = team.tr; w < nwords; w += team.ts) X.vis[w] = 0u;
     // the overlap's size and whether any word was stale; every warp's best
     // seed candidates (a block team takes the one it needs after the barrier)
@@ -558,6 +562,7 @@ __device__ __forceinline__ int icm_pair(const EngineArgs& A, const BlockCtx& B, 
                 sA[i] = (int8_t)-a;
                 if (fA) fA[i] = -fA[i];
             }
+            if (share && has_h) dEa -= 2 * bh[i] * pub_site(pubA, i);
             d[i] ^= 1;
         }
         cnt = n - cnt;
@@ -1085,10 +1090,17 @@ __device__ __forceinline__ int icm_pair(const EngineArgs& A, const BlockCtx& B, 
             int sa = 0, sb = 0;   // spins before the flip
             if (locA) sa = sA[u];
             if (locB) sb = sB[u];
+            if (share) {
+                sb = pub_site(pubB, u);
+                sa = -sb;   // (u is in the overlap)
+            }
             if (by_warp) __syncwarp();
             if (lane == 0) {
-                if (locA) { sA[u] = (int8_t)-sa; dEa -= 2 * sa * hu; }
-                if (locB) { sB[u] = (int8_t)-sb; dEb -= 2 * sb * hu; }
+                if (locA) sA[u] = (int8_t)-sa;
+                if (locB) sB[u] = (int8_t)-sb;
+                if (share) atomicOr(X.vis + (u >> 5), 1u << (u & 31));
+                if (locA || share) dEa -= 2 * sa * hu;
+                if (locB || share) dEb -= 2 * sb * hu;
             }
             const int e1 = brow[u + 1], da = by_warp ? 32 : 1;
 #pragma unroll 4
@@ -1099,9 +1111,9 @@ __device__ __forceinline__ int icm_pair(const EngineArgs& A, const BlockCtx& B, 
                 if (fA) atomicAdd(fA + v, J * (-2 * sa));
                 if (fB) atomicAdd(fB + v, J * (-2 * sb));
                 if (!d[v]) {
-                    const int sv = locA ? sA[v] : sB[v];
-                    if (locA) dEa -= 2 * J * sa * sv;
-                    if (locB) dEb -= 2 * J * sb * sv;
+                    const int sv = share ? pub_site(pubB, v) : (locA ? sA[v] : sB[v]);
+                    if (locA || share) dEa -= 2 * J * sa * sv;
+                    if (locB || share) dEb -= 2 * J * sb * sv;
                 }
             }
         };
@@ -1115,7 +1127,7 @@ __device__ __forceinline__ int icm_pair(const EngineArgs& A, const BlockCtx& B, 
                 const int u = lst[sbase + t];
                 if ((uf_find((volatile int*)X.queue, u) == fast_root) == fast_eq) flip_push(u, by_warp);
             }
-        } else if (BLOCK && (long long)fsize * 4 > (long long)n) {
+        } else if (BLOCK && !share && (long long)fsize * 4 > (long long)n) {
             // a large cluster: flip, then fields and energies from scratch
             // (gathers, no atomics; the cost does not grow with the cluster)
             for_overlap([&](int u) {
@@ -1160,6 +1172,20 @@ __device__ __forceinline__ int icm_pair(const EngineArgs& A, const BlockCtx& B, 
             if (locA) B.E[rA] += dEa;
             if (locB && cnt > 0) B.E[rB] += dEb;
         }
+    }
+    if (share) {
+        // the sites to flip in A and in B and both energies, each word with
+        // the step's tag
+        for (int w = team.tr; w < nwords; w += team.ts) {
+            const uint32_t f = X.vis[w];
+            st_relaxed_gpu_u64(result + w, ((unsigned long long)tag << 32) | (gflip ? ~f : f));
+            st_relaxed_gpu_u64(result + nwords + w, ((unsigned long long)tag << 32) | f);
+        }
+        if (team.tr == 0) {
+            st_relaxed_gpu_u64(result + 2 * nwords, pub_word(tag, B.E[rA] + dEa));
+            st_relaxed_gpu_u64(result + 2 * nwords + 1, pub_word(tag, B.E[rB] + dEb));
+        }
+        team.sync();   // (the next pair clears the bits)
     }
     if (!(BLOCK && algo == ENGINE_ICM_UNION_FIND && cnt > 0)) {
         // (a block team's union-find reset the list counters after its size
@@ -1212,6 +1238,62 @@ __device__ __forceinline__ int gather_pieces(const int32_t* row, const uint32_t*
         for (int k = 0; k < 8; k++) f += (int)(int8_t)(e[k] & 0xffu) * s[k];
     }
     return f;
+}
+
+// Takes over what the group's blocks worked out for the pairs of this block's
+// replicas: tagged words of the sites to flip and the new energies, eight
+// sites per thread and replica, four replicas' words loaded together.  (Every
+// block has published its results or is working on them: no block waits
+// before its own pairs are out.)
+template <int SPACE>
+__device__ __forceinline__ void apply_pairs(const EngineArgs& A, const BlockCtx& B, int chains_even, uint32_t tag,
+                                            volatile int* abortf) {
+    const InstanceDesc& D = B.D;
+    const int tid = threadIdx.x, T = blockDim.x, n = D.n, nt = D.nt, W = (n + 31) >> 5;
+    const unsigned long long limit = A.wait_limit_ns ? A.wait_limit_ns : kWaitLimitNs;
+    // replica j's result and whether it is the pair's second (null: no pair)
+    auto result_of = [&](int j, bool& second) -> const unsigned long long* {
+        if (j >= D.rpc) return nullptr;
+        const int sl = (int)B.rslot[j], c = sl / nt, kk = nt - 1 - (sl - c * nt);
+        second = c & 1;
+        return kk < D.nc && c < chains_even ? A.icm_pub + (long long)((c >> 1) * D.nc + kk) * A.icm_pub_stride : nullptr;
+    };
+    for (int j0 = 0; j0 < D.rpc; j0 += 4) {
+        const unsigned long long* from[4];
+#pragma unroll
+        for (int x = 0; x < 4; x++) {
+            bool second = false;
+            from[x] = result_of(j0 + x, second);
+            if (from[x] != nullptr) {
+                if (tid < 32) {
+                    unsigned long long w = 0;
+                    if (!poll_tagged(from[x] + 2 * W + second, tid == 0, tag, w, abortf, A.status, limit, 6)) return;
+                    if (tid == 0) B.E[B.r0 + j0 + x] = (long long)(int32_t)(uint32_t)w;
+                }
+                if (second) from[x] += W;
+            }
+        }
+        for (int u0 = tid & ~31; u0 < 4 * W; u0 += T) {
+            const int u = u0 + (tid & 31);
+            unsigned long long w[4] = {0, 0, 0, 0};
+#pragma unroll
+            for (int x = 0; x < 4; x++)
+                if (from[x] != nullptr && u < 4 * W) w[x] = ld_relaxed_gpu_u64(from[x] + (u >> 2));
+#pragma unroll
+            for (int x = 0; x < 4; x++) {
+                if (from[x] == nullptr) continue;
+                const bool late = u < 4 * W && (uint32_t)(w[x] >> 32) != tag;
+                if (__any_sync(0xffffffffu, late) &&
+                    !poll_tagged(from[x] + (late ? u >> 2 : 0), late, tag, w[x], abortf, A.status, limit, 6))
+                    return;
+                const SpinRow<SPACE> sp = spin_row<SPACE>(B, j0 + x);
+                for (uint32_t m = ((uint32_t)w[x] >> (8 * (u & 3))) & 0xffu; m != 0 && u < 4 * W; m &= m - 1) {
+                    const int i = 8 * u + __ffs((int)m) - 1;
+                    if (i < n) sp[i] = (int8_t)-sp[i];
+                }
+            }
+        }
+    }
 }
 
 // The local fields of four interleaved replicas at one site per lane (its list
@@ -2390,15 +2472,37 @@ __global__ void __launch_bounds__((REPLAY || (BLOCKTEAM && !NARROW)) ? 1024 : kN
                 IcmScratch X = icm_scratch(s_icm, npad);
                 if (space_large(SPACE) || (SPACE == SP_ANY && !BLOCKTEAM && !REPLAY && S.icm_split))
                     X.list = reinterpret_cast<int*>(g_icm);
-                for (int j = 0; j < rpc; j++) {
-                    const int sl = (int)B.rslot[j], c = sl / nt, k = sl - c * nt, kk = nt - 1 - k;
-                    if (kk >= D.nc || c >= chains_even) continue;
-                    const int cp = c >> 1;
+                // Large instances: every pair is worked out once, by the block
+                // q mod group whichever it holds, and the owners of its two
+                // replicas read the result.  (Each owner for itself, up to
+                // rpc pairs in a row in the blocks of cold replicas, none in
+                // the others and every pair twice: 294 us a step of N=20000
+                // with 136 pairs on 128 blocks; shared 167 us, the time of
+                // the two pairs that eight of the blocks get.)
+                const bool share = space_large(SPACE) && A.icm_pub != nullptr && D.group > 1 && A.flag_barrier &&
+                                   D.icm_algo == ENGINE_ICM_UNION_FIND && !A.icm_exact && A.icm_force == nullptr;
+                const int e1 = share ? (chains_even >> 1) * D.nc : rpc, de = share ? D.group : 1;
+                for (int e = share ? B.rank : 0; e < e1; e += de) {
+                    int cp, kk;
+                    if (share) {
+                        cp = e / D.nc;
+                        kk = e - cp * D.nc;
+                    } else {
+                        const int sl = (int)B.rslot[e], c = sl / nt;
+                        cp = c >> 1;
+                        kk = nt - 1 - (sl - c * nt);
+                        if (kk >= D.nc || c >= chains_even) continue;
+                    }
+                    const int k = nt - 1 - kk;
                     const int rA = (int)B.slot[(2 * cp) * nt + k], rB = (int)B.slot[(2 * cp + 1) * nt + k];
-                    if ((c & 1) && rA >= B.r0 && rA < B.r0 + rpc) continue;
+                    if (!share && (int)B.rslot[e] >= (2 * cp + 1) * nt && rA >= B.r0 && rA < B.r0 + rpc) continue;
                     icm_pair<true, REPLAY, !REPLAY && (NARROW || !BLOCKTEAM), SPACE, !REPLAY && !BLOCKTEAM>(
-                                                                             A, B, team, cp * D.nc + kk, rA, rB,
-                                                                             step, ls, X, 30, P);
+                        A, B, team, cp * D.nc + kk, rA, rB, step, ls, X, 30, P,
+                        share ? A.icm_pub + (long long)e * A.icm_pub_stride : nullptr);
+                }
+                if (share) {
+                    __syncthreads();
+                    apply_pairs<SPACE>(A, B, chains_even, A.pub_base + (uint32_t)ls, abortf);
                 }
             } else {
                 const int warp = tid >> 5, lane = tid & 31;

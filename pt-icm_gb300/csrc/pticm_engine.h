@@ -118,6 +118,8 @@ struct EngineArgs {
     // +1), at (spin offset of the replica) / 16 + k
     unsigned long long* spins_pub;
     long long spins_pub_half;     // words per half (spin pool size / 16)
+    unsigned long long* icm_pub;  // large instances: per pair, the sites to flip in A and in B as tagged words, and
+    long long icm_pub_stride;     // both energies (words per pair); null: each block works out its own pairs
     long long* energy_pub;        // 2 * total replicas (x kPubStride words with flag_barrier)
     long long energy_pub_half;
     unsigned long long* flips;

@@ -114,6 +114,8 @@ struct pticm_ctx {
     DArr<int32_t> d_fields_out; // fields in the original site order (pticm_get_replicas)
     DArr<uint8_t> d_icm_pool;   // ICM scratch when the replicas live in device memory
     long long icm_stride = 0;
+    DArr<unsigned long long> d_icm_pub;   // per pair what is flipped (large instances)
+    long long icm_pub_stride = 0;
     long long ebound = -1;      // energy_bound(P), once
     DArr<long long> d_icm_force;   // per-pair seeds of pticm_icm_pairs
     // bounded waits: limit (0 = kWaitLimitNs) and the barrier test hook
@@ -554,6 +556,13 @@ int configure(pticm_ctx* c, bool replay) {
                                            : (long long)icm_block_bytes(cfg.teams, c->desc.n_pad);
         const size_t want = (size_t)cfg.group * (size_t)c->icm_stride;
         if (c->d_icm_pool.n != want) CK(c->d_icm_pool.alloc(want));
+        if (cfg.plan.icm_split) {
+            // results of the pairs, one of two replicas each: the sites to
+            // flip in both and two energies
+            c->icm_pub_stride = 2 * ((c->desc.n + 31) / 32) + 2;
+            const size_t words = (size_t)(c->R / 2) * (size_t)c->icm_pub_stride;
+            if (c->d_icm_pub.n != words) CK(c->d_icm_pub.alloc(words));
+        }
     }
     std::vector<int32_t> soff, sched;
     single_instance_schedule(cfg.group, soff, sched);
@@ -614,6 +623,8 @@ EngineArgs make_args(pticm_ctx* c) {
     A.flags = engine_flags(c->P, c->o);
     A.icm_pool = c->d_icm_pool.p;
     A.icm_pool_stride = c->icm_stride;
+    A.icm_pub = c->plan.icm_split ? c->d_icm_pub.p : nullptr;
+    A.icm_pub_stride = c->icm_pub_stride;
     A.wait_limit_ns = c->wait_limit_ns;
     A.bar_phantom = c->bar_phantom;
     if (c->ebound < 0) c->ebound = energy_bound(c->P);

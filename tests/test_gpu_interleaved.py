@@ -46,3 +46,24 @@ def test_states_stay_exact(n, deg, wmax, hub, rpb):
         out.append((s, E, bE))
     for x, y in zip(*out):
         assert np.array_equal(x, y)
+
+
+@pytest.mark.parametrize("n,deg,nt,chains,rpb,nc,h", [
+    (13001, 6, 12, 2, 4, 12, True), (14015, 3, 8, 4, 4, 5, False), (16000, 20, 20, 2, 4, 1, True),
+    (20001, 12, 9, 2, 3, 9, True), (19999, 6, 8, 4, 2, 6, False)])
+def test_shared_pairs_equal_the_owners_own(n, deg, nt, chains, rpb, nc, h):
+    """The cluster does not depend on the search: with the breadth-first search
+    each owner (algo 1) works its pairs out, with union-find (2) the blocks share
+    them."""
+    import pticm
+    p = _problem(n, deg, 1, 0, 2 * n + int(h))
+    out = []
+    for algo in (2, 1):
+        ctx = pticm.Context(p, nt=nt, chains=chains, seed=3, icm=True, replicas_per_block=rpb, icm_algo=algo)
+        ctx.set_ladder(pticm.beta_linspace(0.1, 2.0, nt), nc=nc)
+        ctx.init_states(5)
+        ctx.run(9)
+        assert ctx.verify() == 0
+        out.append(ctx.replicas())
+    for a, b in zip(*out):
+        assert np.array_equal(a, b)
