@@ -1301,30 +1301,32 @@ __device__ __forceinline__ void apply_pairs(const EngineArgs& A, const BlockCtx&
 // a quarter of the list's 16-byte pieces, so that a group's loads are whole
 // sectors of one list; one 32-bit load brings a neighbour's spin in all four
 // replicas.  What bounds it is that load's bank conflicts and the lists' way
-// from L2: 215 us a sweep of N=20000, degree 40, 4 replicas on each of 128
+// from L2: 176 us a sweep of N=20000, degree 40, 4 replicas on each of 128
 // SMs.  (One thread per site and a byte load per replica, four times the
-// shared wavefronts and an L1 lookup per lane and piece: 413 us; without the
-// pieces loaded ahead: 267 us.)
+// shared wavefronts and an L1 lookup per lane and piece: 413 us; pieces loaded
+// two at a time when they are needed: 52 us more; at the start of each 32
+// sites only: 13 us more.)
 // PACKED (no field beyond +-127): with the four spins as signed digits of a
 // 32-bit number, base 256, one multiply-add sums all four fields, modulo 2^32;
 // the digits are taken apart at the end.
-// The first kAhead pieces of all four sites are loaded before the first is
-// used: a warp waits for L2 once per 32 sites.
+// The first kAhead pieces of the four sites are in registers already; as each
+// site is done, those of the site that the warp visits next take their place,
+// across the colour classes (lists don't change): L2 answers behind the sums.
+constexpr int kAhead = 3;
+// (of the site of the s-th lane in each group of four)
+__device__ __forceinline__ void load_ahead(const uint32_t* adj, int s, int my0, int my_deg, uint4 (&ahead)[kAhead]) {
+    const int lane = threadIdx.x & 31, src = (lane & ~3) + s;
+    const uint4* const adj4 = reinterpret_cast<const uint4*>(adj);
+    const int e0 = __shfl_sync(0xffffffffu, my0, src), deg = __shfl_sync(0xffffffffu, my_deg, src);
+    const int p0 = (e0 >> 2) + (lane & 3), p1 = (e0 + deg + 3) >> 2;
+#pragma unroll
+    for (int x = 0; x < kAhead; x++) ahead[x] = p0 + 4 * x < p1 ? adj4[p0 + 4 * x] : make_uint4(0, 0, 0, 0);
+}
 template <bool PACKED>
-__device__ __forceinline__ void gather4(const uint32_t* adj, const uint32_t* s4, int my0, int my_deg, int (&f)[4]) {
-    constexpr int kAhead = 3;
+__device__ __forceinline__ void gather4(const uint32_t* adj, const uint32_t* s4, int my0, int my_deg, int next0,
+                                        int next_deg, uint4 (&ahead)[4][kAhead], int (&f)[4]) {
     const int lane = threadIdx.x & 31, sub = lane & 3;
     const uint4* const adj4 = reinterpret_cast<const uint4*>(adj);
-    uint4 ahead[4][kAhead];
-#pragma unroll
-    for (int s = 0; s < 4; s++) {
-        const int src = (lane & ~3) + s;
-        const int e0 = __shfl_sync(0xffffffffu, my0, src), deg = __shfl_sync(0xffffffffu, my_deg, src);
-        const int p0 = (e0 >> 2) + sub, p1 = (e0 + deg + 3) >> 2;
-#pragma unroll
-        for (int x = 0; x < kAhead; x++)
-            ahead[s][x] = p0 + 4 * x < p1 ? adj4[p0 + 4 * x] : make_uint4(0, 0, 0, 0);
-    }
 #pragma unroll
     for (int s = 0; s < 4; s++) {
         const int src = (lane & ~3) + s;
@@ -1352,6 +1354,7 @@ __device__ __forceinline__ void gather4(const uint32_t* adj, const uint32_t* s4,
         };
 #pragma unroll
         for (int x = 0; x < kAhead; x++) piece(ahead[s][x], p0 + 4 * x);
+        load_ahead(adj, s, next0, next_deg, ahead[s]);
 #pragma unroll 1
         for (int p = p0 + 4 * kAhead; p < p1; p += 4) piece(adj4[p], p);
         if (PACKED) {
@@ -1423,6 +1426,32 @@ __device__ void colored_sweep(const EngineArgs& A, const BlockCtx& B, unsigned l
     const int32_t* const h1 = B.h;
     const uint32_t* const thr1 = ONE ? s_thr + B.tb[0] : s_thr;
     const int ncolors = D.ncolors;
+    // interleaved replicas: the warp's 32 sites now and next (their class,
+    // first site and lists), and list pieces loaded ahead
+    struct Sites { int c, base, e0, deg; } at{}, next{};
+    uint4 ahead[4][kAhead];
+    auto advance = [&](Sites& x) {
+        x.base += T;
+        while (x.c < ncolors && x.base >= s_col[x.c + 1]) {
+            if (++x.c < ncolors) x.base = s_col[x.c] + (tid & ~31);
+        }
+        const int i = x.base + lane;
+        x.e0 = x.deg = 0;
+        if (x.c < ncolors && i < s_col[x.c + 1]) {
+            x.e0 = row[i];
+            x.deg = row[i + 1] - x.e0;
+        }
+    };
+    ThreadRngWindow rng4;
+    if (SPACE == SP_LARGE4) {
+        rng4.start(stream_key(A.seed, STREAM_SWEEP), (uint32_t)(B.rank * T + tid), sweep_idx, (uint32_t)D.inst_id << 16);
+        at.base = s_col[0] + (tid & ~31) - T;
+        advance(at);
+        next = at;
+        advance(next);
+#pragma unroll
+        for (int s = 0; s < 4; s++) load_ahead(adj, s, at.e0, at.deg, ahead[s]);
+    }
     for (int c = 0; c < ncolors; c++) {
         const int c0 = s_col[c];
         const int Sc = s_col[c + 1] - c0;
@@ -1540,42 +1569,48 @@ __device__ void colored_sweep(const EngineArgs& A, const BlockCtx& B, unsigned l
             int g_de[4] = {0, 0, 0, 0};
             unsigned g_fl[4] = {0, 0, 0, 0};
             uint32_t* const s4 = reinterpret_cast<uint32_t*>(B.spin);
-            int e0 = 0, deg = 0;   // (of the site after this one)
-            auto list_of = [&](int i) {
-                e0 = 0;
-                deg = 0;
-                if (i < c0 + Sc) {
-                    e0 = row[i];
-                    deg = row[i + 1] - e0;
-                }
-            };
-            list_of(c0 + tid);
             for (int base = c0 + (tid & ~31); base < c0 + Sc; base += T) {
                 const int i = base + lane;
                 int f[4];
-                const int a0 = e0, ad = deg;
-                list_of(i + T);
-                if (kmax <= 127) gather4<true>(adj, s4, a0, ad, f);
-                else gather4<false>(adj, s4, a0, ad, f);
-                if (i >= c0 + Sc) continue;
-                const int hi = B.h ? B.h[i] : 0;
-                uint32_t w = s4[i];
-                const uint32_t w0 = w;
+                const int e0 = at.e0, deg = at.deg;
+                at = next;
+                advance(next);
+                if (kmax <= 127) gather4<true>(adj, s4, e0, deg, at.e0, at.deg, ahead, f);
+                else gather4<false>(adj, s4, e0, deg, at.e0, at.deg, ahead, f);
+                const bool have = i < c0 + Sc;
+                const int hi = have && B.h ? B.h[i] : 0;
+                const uint32_t w0 = have ? s4[i] : 0u;
+                uint32_t w = w0;
+                // the four thresholds side by side, then the decisions in
+                // replica order, without a branch (branches and a refill of
+                // twelve words wherever a lane ran out: 245 us a sweep)
+                int de[4];
+                uint32_t thr[4];
 #pragma unroll
                 for (int j = 0; j < 4; j++) {
-                    const int s = (int)(int8_t)(w0 >> (8 * j));
-                    const int de = -2 * s * (f[j] + hi);
-                    bool acc = de <= 0;
-                    if (!acc) {
-                        const uint32_t thr = s_thr[B.tb[j] + min(de >> 1, kmax)];
-                        acc = (rng.next() < thr) || (thr == 0xFFFFFFFFu);
+                    de[j] = have ? -2 * (int)(int8_t)(w0 >> (8 * j)) * (f[j] + hi) : 0;
+                    thr[j] = s_thr[B.tb[j] + min(max(de[j], 0) >> 1, kmax)];
+                }
+                uint32_t u[4];
+                rng4.peek(u);
+                uint32_t drawn = 0;
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    const bool up = de[j] > 0;
+                    const bool acc = have && (!up || u[0] < thr[j] || thr[j] == 0xFFFFFFFFu);
+                    if (up) {
+                        u[0] = u[1];
+                        u[1] = u[2];
+                        u[2] = u[3];
+                        drawn++;
                     }
                     if (acc) {
                         w ^= 0xFEu << (8 * j);   // 0x01 <-> 0xFF
-                        g_de[j] += de;
+                        g_de[j] += de[j];
                         g_fl[j]++;
                     }
                 }
+                rng4.take(drawn);
                 if (w != w0) s4[i] = w;
             }
             __syncwarp();

@@ -177,6 +177,47 @@ struct ThreadRng12 {
     }
 };
 
+// The same stream for a thread that draws up to four words at a time: the
+// Philox block of the next word and the one after it.  Threads of a warp draw
+// at different rates, so a refill on an empty buffer runs in nearly every
+// draw for some lane; here one block at most is computed per four draws, by
+// all lanes that moved on at once.
+struct ThreadRngWindow {
+    uint4 a, b;
+    uint32_t at, calls;   // words of a that are used; the block after b
+    uint4 ctr;
+    uint2 key;
+
+    __device__ __forceinline__ uint4 block(uint32_t call) const {
+        uint4 x = ctr;
+        x.w = call;
+        return philox4x32_10(x, key);
+    }
+    __device__ __forceinline__ void start(uint2 k, uint32_t tid, unsigned long long sweep, uint32_t call0) {
+        key = k;
+        ctr = make_uint4(tid, (uint32_t)sweep, (uint32_t)(sweep >> 32), 0u);
+        a = block(call0);
+        b = block(call0 + 1);
+        calls = call0 + 2;
+        at = 0;
+    }
+    // the next four words
+    __device__ __forceinline__ void peek(uint32_t (&u)[4]) const {
+        const bool two = at & 2u, one = at & 1u;
+        const uint32_t x[5] = {two ? a.z : a.x, two ? a.w : a.y, two ? b.x : a.z, two ? b.y : a.w, two ? b.z : b.x};
+#pragma unroll
+        for (int q = 0; q < 4; q++) u[q] = one ? x[q + 1] : x[q];
+    }
+    __device__ __forceinline__ void take(uint32_t count) {   // at most four
+        at += count;
+        if (at >= 4) {
+            at -= 4;
+            a = b;
+            b = block(calls++);
+        }
+    }
+};
+
 // Uniform in (0, 1] from the top 24 bits (never zero, so log() is finite).
 __device__ __forceinline__ float u01_open0(uint32_t x) {
     return ((float)(x >> 8) + 1.0f) * (1.0f / 16777216.0f);
