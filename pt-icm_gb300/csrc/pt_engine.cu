@@ -1443,8 +1443,9 @@ __device__ void colored_sweep(const EngineArgs& A, const BlockCtx& B, unsigned l
         }
     };
     ThreadRngWindow rng4;
-    if (SPACE == SP_LARGE4) {
+    if (SPACE == SP_LARGE4 || (!ONE && !gm))
         rng4.start(stream_key(A.seed, STREAM_SWEEP), (uint32_t)(B.rank * T + tid), sweep_idx, (uint32_t)D.inst_id << 16);
+    if (SPACE == SP_LARGE4) {
         at.base = s_col[0] + (tid & ~31) - T;
         advance(at);
         next = at;
@@ -1701,40 +1702,76 @@ __device__ void colored_sweep(const EngineArgs& A, const BlockCtx& B, unsigned l
         } else {
             const int items = rpc * Sc;
             const int items_w = (items + 31) & ~31;   // whole warps iterate together
-            for (int it = tid; it < items_w; it += T) {
-                int j = -1, de = 0;
-                bool acc = false;
-                if (it < items) {
-                    j = it / Sc;
-                    const int i = c0 + (it - j * Sc);
-                    int8_t* sp = B.spin + j * npad;
-                    int32_t* fd = B.field ? B.field + j * npad : nullptr;
-                    const int s = sp[i];
-                    const int f = (fd ? fd[i] : gather_field(row, adj, sp, i)) + (B.h ? B.h[i] : 0);
-                    de = -2 * s * f;
-                    acc = de <= 0;
-                    if (!acc) {
-                        const uint32_t thr = s_thr[B.tb[j] + min(de >> 1, kmax)];
-                        acc = (rng.next() < thr) || (thr == 0xFFFFFFFFu);
+            // (item it: replica jt, site ct of the class; two divisions a
+            // class instead of one an item)
+            const int Sd = max(Sc, 1), jd = T / Sd, cd = T - jd * Sd;
+            int jt = tid / Sd, ct = tid - jt * Sd;
+            // four items of a thread at a time (sites of one class share no
+            // edge, so none sees another's flip): their loads overlap, and
+            // their draws take at most one Philox block
+            for (int it = tid; it < items_w; it += 4 * T) {
+                int jx[4], ix[4], sx[4], de[4];
+                uint32_t thr[4];
+#pragma unroll
+                for (int x = 0; x < 4; x++) {
+                    const bool have = it + x * T < items;
+                    jx[x] = have ? jt : 0;
+                    ix[x] = c0 + (have ? ct : 0);
+                    const int8_t* sp = B.spin + jx[x] * npad;
+                    sx[x] = have ? sp[ix[x]] : 0;
+                    const int f = (B.field ? B.field[jx[x] * npad + ix[x]] : have ? gather_field(row, adj, sp, ix[x]) : 0) +
+                                  (B.h ? B.h[ix[x]] : 0);
+                    de[x] = -2 * sx[x] * f;
+                    jt += jd;
+                    ct += cd;
+                    if (ct >= Sd) {
+                        ct -= Sd;
+                        jt++;
                     }
-                    if (acc) {
-                        sp[i] = (int8_t)-s;
-                        if (fd) {
-                            const int dl = -2 * s;
-                            for_each_neighbour(row, adj, i, [&](uint32_t e) {
+                }
+#pragma unroll
+                for (int x = 0; x < 4; x++) thr[x] = s_thr[B.tb[jx[x]] + min(max(de[x], 0) >> 1, kmax)];
+                uint32_t u[4], drawn = 0;
+                rng4.peek(u);
+                bool acc[4];
+#pragma unroll
+                for (int x = 0; x < 4; x++) {
+                    const bool up = de[x] > 0;
+                    acc[x] = sx[x] != 0 && (!up || u[0] < thr[x] || thr[x] == 0xFFFFFFFFu);
+                    if (up) {
+                        u[0] = u[1];
+                        u[1] = u[2];
+                        u[2] = u[3];
+                        drawn++;
+                    }
+                }
+                rng4.take(drawn);
+#pragma unroll
+                for (int x = 0; x < 4; x++) {
+                    if (acc[x]) {
+                        B.spin[jx[x] * npad + ix[x]] = (int8_t)-sx[x];
+                        if (B.field) {
+                            int32_t* const fd = B.field + jx[x] * npad;
+                            const int dl = -2 * sx[x];
+                            for_each_neighbour(row, adj, ix[x], [&](uint32_t e) {
                                 atomicAdd(fd + (e >> 8), (int)(int8_t)(e & 0xffu) * dl);
                             });
                         }
                     }
-                }
-                // one shared-memory update per replica per warp instead of per flip
-                const int key = acc ? j : -1;
-                const unsigned grp = __match_any_sync(0xffffffffu, key);
-                if (acc) {
-                    const int sde = __reduce_add_sync(grp, de);
-                    if (lane == __ffs(grp) - 1) {
-                        atomicAdd(s_dEp + j, sde);
-                        atomicAdd(s_flp + j, (unsigned)__popc(grp));
+                    // one shared-memory update per replica per warp instead of
+                    // per flip (the items of a warp lie in one replica, or in
+                    // a few neighbouring ones: its lanes' sums by replica)
+                    unsigned left = __ballot_sync(0xffffffffu, acc[x]);
+                    while (left) {
+                        const int jj = __shfl_sync(0xffffffffu, jx[x], __ffs(left) - 1);
+                        const bool mine = acc[x] && jx[x] == jj;
+                        const unsigned grp = __ballot_sync(0xffffffffu, mine);
+                        const int sde = (int)__reduce_add_sync(0xffffffffu, mine ? (unsigned)de[x] : 0u);
+                        if (lane == 0) {
+                            atomicAdd(s_dEp + jj, sde);
+                            atomicAdd(s_flp + jj, (unsigned)__popc(grp));
+                        }
+                        left &= ~grp;
                     }
                 }
             }
