@@ -246,7 +246,7 @@ int configure_batch(pticm_batch* b) {
     int dev = 0, sms = 0, per_sm = 0;
     BCK(cudaGetDevice(&dev));
     BCK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    BCK(engine_max_blocks_per_sm(false, false, false, b->threads, b->plan.total, &per_sm));
+    BCK(engine_max_blocks_per_sm(false, false, false, b->threads, b->plan, &per_sm));
     if (per_sm < 1) return bfail(PTICM_ERR_UNSUPPORTED, "the engine block does not fit on an SM");
     long long total_blocks = 0;
     int gmax = 0;

@@ -2879,21 +2879,20 @@ cudaError_t launch_engine(const EngineArgs& A0, int threads, bool replay, bool b
     return cudaLaunchKernel(fn, dim3(A.n_blocks), dim3(threads), args, A.sm.total, stream);
 }
 
-cudaError_t engine_max_blocks_per_sm(bool replay, bool block_team, bool narrow, int threads, size_t smem, int* out) {
-    if (!replay && (narrow || !block_team) && threads > kNarrowThreads) {
-        *out = 0;
-        return cudaSuccess;
-    }
-    // the launch takes one of the variants by its plan: what all of them hold
-    *out = 1 << 20;
-    for (int space : {SP_ANY, SP_SHARED, SP_STATE, SP_LARGE, SP_LARGE4}) {
-        const void* fn = engine_fn(replay, block_team, narrow, space);
-        cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        int per_sm = 0;
-        if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, smem);
-        if (e != cudaSuccess) return e;
-        *out = std::min(*out, per_sm);
-    }
+// Blocks per SM of the variant that a launch with this plan takes (only that
+// one is loaded: a variant costs a new process 10-20 ms).  Layouts must not
+// depend on how many registers a variant came out with, so the narrow ones
+// count as their bound of 128.
+cudaError_t engine_max_blocks_per_sm(bool replay, bool block_team, bool narrow, int threads, const SmemPlan& S, int* out) {
+    *out = 0;
+    const bool bounded = !replay && (narrow || !block_team);
+    if (bounded && threads > kNarrowThreads) return cudaSuccess;
+    const void* fn = engine_fn(replay, block_team, narrow, plan_space(S, block_team));
+    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S.total);
+    int per_sm = 0;
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, S.total);
+    if (e != cudaSuccess) return e;
+    *out = bounded ? std::min(per_sm, 65536 / (128 * ((threads + 31) & ~31))) : per_sm;
     return cudaSuccess;
 }
 

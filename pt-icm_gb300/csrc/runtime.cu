@@ -308,7 +308,7 @@ int choose_config(const HostProblem& P, const pticm_opts& o, bool replay, Instan
                 const SmemPlan p1 = make_plan(d1, false, 1, t, false, false, true, split);
                 int per_sm = 0;
                 if (p1.total > kSmemLimit ||
-                    engine_max_blocks_per_sm(false, false, false, t, p1.total, &per_sm) != cudaSuccess ||
+                    engine_max_blocks_per_sm(false, false, false, t, p1, &per_sm) != cudaSuccess ||
                     (int64_t)per_sm * sms < R / rp)
                     continue;
                 rpc = rp;
@@ -333,7 +333,7 @@ int choose_config(const HostProblem& P, const pticm_opts& o, bool replay, Instan
                 const SmemPlan p1 = make_plan(d1, false, 1, t, false, false, true);
                 if (p1.total > kSmemLimit) continue;
                 int per_sm = 0;
-                if (engine_max_blocks_per_sm(false, true, false, t, p1.total, &per_sm) != cudaSuccess) continue;
+                if (engine_max_blocks_per_sm(false, true, false, t, p1, &per_sm) != cudaSuccess) continue;
                 if ((int64_t)per_sm * sms < R) continue;
                 rpc = 1;
                 threads = t;
@@ -371,7 +371,7 @@ int choose_config(const HostProblem& P, const pticm_opts& o, bool replay, Instan
                 const SmemPlan p1 = make_plan(d1, false, 1, t, false, true);
                 if (p1.total > kSmemLimit) continue;
                 int per_sm = 0;
-                if (engine_max_blocks_per_sm(false, true, false, t, p1.total, &per_sm) != cudaSuccess) continue;
+                if (engine_max_blocks_per_sm(false, true, false, t, p1, &per_sm) != cudaSuccess) continue;
                 if ((int64_t)per_sm * sms < R) continue;
                 rpc = 1;
                 threads = t;
@@ -402,7 +402,7 @@ int choose_config(const HostProblem& P, const pticm_opts& o, bool replay, Instan
     bool narrow = false;
     if (block_team && threads <= kNarrowThreads) {
         int per_sm = 0;
-        if (engine_max_blocks_per_sm(false, true, true, threads, plan.total, &per_sm) == cudaSuccess &&
+        if (engine_max_blocks_per_sm(false, true, true, threads, plan, &per_sm) == cudaSuccess &&
             (int64_t)per_sm * sms >= group)
             narrow = true;
     }
@@ -418,7 +418,7 @@ int choose_config(const HostProblem& P, const pticm_opts& o, bool replay, Instan
     cfg.plan = plan;
     if (group > 1) {
         int per_sm = 0;
-        e = engine_max_blocks_per_sm(replay, block_team, narrow, threads, plan.total, &per_sm);
+        e = engine_max_blocks_per_sm(replay, block_team, narrow, threads, plan, &per_sm);
         if (e != cudaSuccess) { msg = cudaGetErrorString(e); return PTICM_ERR_CUDA; }
         if ((int64_t)per_sm * sms < group) {
             msg = "the replica blocks of one instance cannot all be resident (" + std::to_string(group) +
