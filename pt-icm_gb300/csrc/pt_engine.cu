@@ -1827,7 +1827,7 @@ __device__ void colored_sweep(const EngineArgs& A, const BlockCtx& B, unsigned l
 // replica: lane 0 makes each decision exactly as src/replica.cc:31-38 does
 // (dE <= 0, else u < exp(-beta*dE) with a recorded u), the warp applies the
 // field update and copies a new best state (src/replica.cc:18-29).
-__device__ void replay_sweep(const EngineArgs& A, const BlockCtx& B, int ls, int sw,
+static __device__ void replay_sweep(const EngineArgs& A, const BlockCtx& B, int ls, int sw,
                              unsigned long long sweep_idx, const double* s_ptab,
                              unsigned long long* s_flips, long long* s_bestE) {
     const InstanceDesc& D = B.D;
@@ -1926,7 +1926,7 @@ __device__ __forceinline__ bool swap_accepted(double dbeta, long long dE, float 
 // took 8.2 us for 20 pairs and two chains.)
 constexpr uint32_t kWaitLeft = 1u << 30, kWaitRight = 1u << 31, kPosBits = 24;
 
-__device__ void exchange_reference_draw(const EngineArgs& A, const InstanceDesc& D, unsigned long long step,
+static __device__ void exchange_reference_draw(const EngineArgs& A, const InstanceDesc& D, unsigned long long step,
                                         float* s_xlogu, uint32_t* s_xrand) {
     const int total = D.chains * (D.nt - 1), ndraw = 2 * total;
     const uint2 key = stream_key(A.seed, STREAM_EXCHANGE);
@@ -1949,7 +1949,7 @@ __device__ void exchange_reference_draw(const EngineArgs& A, const InstanceDesc&
 // an earlier attempt on the pair below or above goes to the same chain.
 // s_pos: each pair's position after all passes' reshuffles, which the exchange
 // makes the order.
-__device__ void exchange_reference_plan(const InstanceDesc& D, const uint32_t* s_order, uint32_t* s_xrand,
+static __device__ void exchange_reference_plan(const InstanceDesc& D, const uint32_t* s_order, uint32_t* s_xrand,
                                         uint32_t* s_pos, int* s_next) {
     const int lane = threadIdx.x & 31, C = D.chains, m = D.nt - 1;
     for (int i = lane; i < m; i += 32) s_pos[s_order[i]] = (uint32_t)i;
@@ -1988,7 +1988,7 @@ __device__ void exchange_reference_plan(const InstanceDesc& D, const uint32_t* s
     }
 }
 
-__device__ void exchange_reference_order(const BlockCtx& B, const double* s_dbeta, unsigned* s_att, unsigned* s_succ,
+static __device__ void exchange_reference_order(const BlockCtx& B, const double* s_dbeta, unsigned* s_att, unsigned* s_succ,
                                          const float* s_xlogu, const uint32_t* s_xrand, const uint32_t* s_pos,
                                          uint32_t* s_order, int* s_done, const Prof P) {
     const InstanceDesc& D = B.D;
@@ -2098,7 +2098,7 @@ __device__ __forceinline__ EvenOddDraws even_odd_draw(const EngineArgs& A, const
 
 // Deterministic even/odd exchange: per chain, all even pairs, then all odd
 // pairs, each set in parallel (nt-1 attempts per chain per step).
-__device__ void exchange_even_odd(const EngineArgs& A, const BlockCtx& B, unsigned long long step,
+static __device__ void exchange_even_odd(const EngineArgs& A, const BlockCtx& B, unsigned long long step,
                                   const double* s_dbeta, unsigned* s_att, unsigned* s_succ, EvenOddDraws u) {
     const InstanceDesc& D = B.D;
     const int tid = threadIdx.x, T = blockDim.x;
@@ -2129,7 +2129,7 @@ __device__ void exchange_even_odd(const EngineArgs& A, const BlockCtx& B, unsign
 
 // Replayed exchange: the recorded pair sequence and log-uniforms, applied
 // sequentially in FP64 exactly as src/replica_exchange.cc:20-40 computes.
-__device__ void exchange_replay(const EngineArgs& A, const BlockCtx& B, int ls, const double* s_beta,
+static __device__ void exchange_replay(const EngineArgs& A, const BlockCtx& B, int ls, const double* s_beta,
                                 unsigned* s_att, unsigned* s_succ) {
     const InstanceDesc& D = B.D;
     if (threadIdx.x == 0) {
@@ -2638,6 +2638,17 @@ __global__ void __launch_bounds__((REPLAY || (BLOCKTEAM && !NARROW)) ? 1024 : kN
     }
 }
 
+// The variants for blocks of several replicas (their own object file,
+// pt_engine_multi.cu: eight variants in one take two minutes to compile).
+void* engine_fn_multi(int space);
+#ifdef PTICM_ENGINE_MULTI
+void* engine_fn_multi(int space) {
+    if (space == SP_SHARED || space == SP_STATE) return (void*)pt_engine_kernel<false, false, false, SP_STATE>;
+    if (space == SP_LARGE) return (void*)pt_engine_kernel<false, false, false, SP_LARGE>;
+    if (space == SP_LARGE4) return (void*)pt_engine_kernel<false, false, false, SP_LARGE4>;
+    return (void*)pt_engine_kernel<false, false, false, SP_ANY>;
+}
+#else
 // --------------------------------------------------- from-scratch checks
 // For every replica: fields f_i = sum_j J_ij s_j, E = sum h s + 1/2 sum s f
 // and the cut sum over edges of w [s_i != s_j] (src/problem.cc:33-162),
@@ -2845,10 +2856,7 @@ static void* engine_fn(bool replay, bool block_team, bool narrow, int space) {
         return space == SP_SHARED ? (void*)pt_engine_kernel<false, true, true, SP_SHARED>
                                   : (void*)pt_engine_kernel<false, true, true, SP_ANY>;
     if (block_team) return (void*)pt_engine_kernel<false, true, false, SP_ANY>;
-    if (space == SP_SHARED || space == SP_STATE) return (void*)pt_engine_kernel<false, false, false, SP_STATE>;
-    if (space == SP_LARGE) return (void*)pt_engine_kernel<false, false, false, SP_LARGE>;
-    if (space == SP_LARGE4) return (void*)pt_engine_kernel<false, false, false, SP_LARGE4>;
-    return (void*)pt_engine_kernel<false, false, false, SP_ANY>;
+    return engine_fn_multi(space);
 }
 
 // The address spaces of a plan's launch.  (A staged plan of one instance
@@ -2951,5 +2959,7 @@ cudaError_t launch_philox_probe(const uint4* ctr, const uint2* key, uint4* out, 
     philox_probe_kernel<<<(count + 127) / 128, 128, 0, stream>>>(ctr, key, out, count);
     return cudaGetLastError();
 }
+
+#endif  // PTICM_ENGINE_MULTI
 
 }  // namespace pticm

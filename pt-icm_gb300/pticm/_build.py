@@ -26,7 +26,7 @@ NVFLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC,-ffp-contract=
            "--expt-relaxed-constexpr"] + ARCH
 INCS = ["-I", os.path.join(REPO, "include"), "-I", CSRC]
 
-LIB_SOURCES = ["pt_engine.cu", "runtime.cu", "problem_host.cc", "noalloc.cu", "replica.cu", "smem_rate.cu", "mhist.cu", "mhist_host.cc", "tc_gemm.cu", "mlp.cu", "mlp_fused.cu", "batch.cu", "surrogate.cu"]
+LIB_SOURCES = ["pt_engine.cu", "pt_engine_multi.cu", "runtime.cu", "problem_host.cc", "noalloc.cu", "replica.cu", "smem_rate.cu", "mhist.cu", "mhist_host.cc", "tc_gemm.cu", "mlp.cu", "mlp_fused.cu", "batch.cu", "surrogate.cu"]
 
 
 def nvcc() -> str:
@@ -51,7 +51,7 @@ def _newest_input(src: str) -> float:
     t = os.path.getmtime(src)
     for d in (CSRC, os.path.join(REPO, "include")):
         for f in os.listdir(d):
-            if f.endswith((".h", ".cuh", ".hh")):
+            if f.endswith((".h", ".cuh", ".hh")) or (src.endswith("pt_engine_multi.cu") and f == "pt_engine.cu"):
                 t = max(t, os.path.getmtime(os.path.join(d, f)))
     return t
 
