@@ -40,8 +40,8 @@ namespace cg = cooperative_groups;
 // two matrix-vector products and no exponential: 10.4 ms instead of 504 ms, 7.8
 // us an iteration over 16 SMs (the two products about 3 us of FP64 pipe, the
 // rest the divisions, the sums' short chains and the cluster's barrier).
-// Against extended precision ln g is off by 1e-16 of its scale, the
-// exponentials of every iteration's a_j were off by 1e-14.  The reference moves to the
+// Against extended precision ln g is off by 2e-16 of its scale, the
+// exponentials of every iteration's a_j were off by up to 8e-14.  The reference moves to the
 // current a_j when an x_j leaves [e^-20, e^20] (27 times in those 1338
 // iterations).  K_ij below e^-120 is zero: with every |ln x_j| at most 35 the
 // dropped terms of S_i are below e^-50 of it, and of T_j below e^-65.
