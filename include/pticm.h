@@ -218,6 +218,12 @@ typedef struct pticm_layout {
 } pticm_layout;
 PTICM_API int pticm_get_layout(pticm_ctx* c, pticm_layout* out);
 
+/* The sweep and the cluster search chosen with the layout: threads that
+ * gather one site's field from its neighbours' spins (0: the fields are
+ * stored, or gathered by another layout's rule), and whether the cluster
+ * search unites along every edge (1) or samples links first (0). */
+PTICM_API int pticm_get_paths(pticm_ctx* c, uint32_t* field_lanes, uint32_t* all_edges);
+
 /* Ladder and slot -> replica map (beta_indices of src/replica_exchange.cc). */
 PTICM_API int pticm_get_ladder(pticm_ctx* c, double* beta, uint32_t* slot_to_replica, uint32_t* nc);
 

@@ -468,6 +468,7 @@ int pticm_batch_create(const pticm_problem* const* problems, uint32_t count, con
         D.has_h = P.has_h ? 1 : 0;
         D.inst_id = (int32_t)i;
         D.icm_algo = engine_flags(P, *o) & ENGINE_ICM_MASK;
+        D.all_edges = icm_all_edges(P) ? 1 : 0;
         // every segment starts on 16 bytes: the adjacency is staged by bulk
         // copies, which need 16-byte aligned global addresses
         D.row_off = (int64_t)row.size();

@@ -202,16 +202,6 @@ struct SpinRow {
     __device__ __forceinline__ int8_t& operator[](int i) const { return p[space_stride(SPACE) * i]; }
 };
 
-// The cluster search unites along every edge, instead of sampling links first,
-// for few neighbours, few colour classes (two or three: the sites of one class
-// all hook under sites of the others, so the trees stay shallow) and few sites
-// per thread: on the +-1 lattice of 400 sites the search takes 3.3 us against
-// 5.6 (step 15.3 -> 12.7 us), of 1764 sites the step 1.2 times less; with mean
-// degree 8 it takes 5.5 against 4.8, and on a random graph of 15515 sites and
-// degree 4.7 the unions' walks to the giant component's root made the step
-// 2.8 times longer.
-constexpr int kDirectDegree = 5, kDirectSites = 2560;
-
 // Per-block view of a job: its descriptor (in shared memory) and pointers,
 // which are shared-memory offsets of the launch's plan or device addresses.
 struct BlockCtx {
@@ -676,7 +666,7 @@ __device__ __forceinline__ int icm_pair(const EngineArgs& A, const BlockCtx& B, 
                 team.sync();
             }
             // (few neighbours: every edge is a link, nothing to sample)
-            const bool direct = algo == ENGINE_ICM_UNION_FIND && D.nnz <= kDirectDegree * n && n <= kDirectSites && D.ncolors <= 3;
+            const bool direct = algo == ENGINE_ICM_UNION_FIND && D.all_edges != 0;
             if (direct) {
                 // every edge from its upper end: each site is hooked under
                 // its lowest overlap neighbour below it by a plain store,

@@ -35,6 +35,8 @@ struct InstanceDesc {
     int32_t stage;      // 1: adjacency staged into shared memory by bulk copy
     int32_t teams;      // ICM warp teams of a block (scratch of icm_team_bytes(n_pad) each)
     int32_t lanes;      // threads that gather one site's field in a narrow block team's sweep (power of two, <= 32)
+    int32_t all_edges;  // 1: the union-find cluster search unites along every edge instead of sampling links first
+    int32_t pad0;
     int64_t row_off;    // int32 pool: n+1 row starts (relative to the instance)
     int64_t adj_off;    // uint32 pool: nnz packed entries (col << 8 | (uint8)J)
     int64_t col_off;    // int32 pool: ncolors+1 colour-class starts

@@ -492,12 +492,46 @@ static int gather_lanes(const HostProblem& P, int threads) {
     return best;
 }
 
+// The cluster search unites along every edge, instead of sampling links first,
+// for few neighbours (mean degree up to five: of eight, it takes 5.5 us against
+// 4.8 on 400 sites) and two or three colour classes: the sites of one class all
+// hook under sites of the others, so that the trees stay shallow.  On the +-1
+// lattice of 400 sites the step takes 11.2 us against 14.1, of 2500 sites 22.4
+// against 29.7.
+// A list goes to one thread, twice, whose unions follow one another; sampling
+// stops at the second overlap neighbour and skips the giant component.  So not
+// with more than a twentieth of all list entries in lists longer than
+// kDirectList (two links per site by preferential attachment: 400 sites, a
+// list of 66, 25.8 us against 16.3; 2500 sites 81.5 against 25.6; a lattice of
+// 961 sites with one list of 32: 15.1 against 18.9).  And past kDirectAny
+// sites, where random graphs' unions walk to the giant component's root (degree
+// 3 or 4: 1000 sites 15.0 against 17.5, 1200 sites 0.87 to 1.03 times the
+// sampled step, 1400 sites up to 1.43, 2500 sites 32.2 against 23.4), only
+// lattice-like lists or close to two neighbours (2200 sites, degree 2.2: 24.3
+// against 24.5; 2.5: 26.8 against 22.9).  Lattices past kDirectSites, which
+// are sampled, would gain as well (10000 sites: 76 against 116 us).
+constexpr int kDirectDegree = 5, kDirectSites = 2560, kDirectAny = 1200, kDirectList = 16, kLatticeList = 4;
+
+bool icm_all_edges(const HostProblem& P) {
+    const int64_t nnz = (int64_t)P.dadj.size();
+    if (nnz > kDirectDegree * P.n || P.n > kDirectSites || P.ncolors > 3) return false;
+    int64_t in_long = 0, longest = 0;
+    for (int64_t i = 0; i < P.n; i++) {
+        const int64_t len = P.drow[i + 1] - P.drow[i];
+        longest = std::max(longest, len);
+        if (len > kDirectList) in_long += len;
+    }
+    if (20 * in_long > nnz) return false;
+    return P.n <= kDirectAny || longest <= kLatticeList || 4 * nnz <= 9 * P.n;
+}
+
 void finish_desc(InstanceDesc& D, const HostProblem& P, const pticm_opts& o, const LaunchConfig& cfg) {
     const double degree = (double)P.dadj.size() / (double)std::max<int64_t>(P.n, 1);
     const bool gather = cfg.narrow && (degree <= kGatherUpTo || cfg.field_gather ||
                                        (cfg.plan.stage_adj && (D.nc == 0 || degree >= kGatherFrom)));
     D.lanes = gather ? gather_lanes(P, cfg.threads) : 0;
     D.icm_algo = engine_flags(P, o) & ENGINE_ICM_MASK;
+    D.all_edges = icm_all_edges(P) ? 1 : 0;
     D.stage = cfg.plan.stage_adj;
     D.rpc = cfg.rpc;
     D.group = cfg.group;
@@ -1214,6 +1248,14 @@ int pticm_get_layout(pticm_ctx* c, pticm_layout* out) {
     out->narrow = c->narrow ? 1 : 0;
     out->adjacency_staged = c->plan.stage_adj;
     out->state_mode = c->plan.state_global ? 2 : (c->plan.field_gather ? 1 : 0);
+    return PTICM_OK;
+}
+
+int pticm_get_paths(pticm_ctx* c, uint32_t* field_lanes, uint32_t* all_edges) {
+    if (!c || !field_lanes || !all_edges) return fail(PTICM_ERR_INVALID, "null argument");
+    if (!c->configured) return fail(PTICM_ERR_INVALID, "the layout is chosen with the first states");
+    *field_lanes = (uint32_t)c->desc.lanes;
+    *all_edges = c->desc.all_edges && c->desc.icm_algo == ENGINE_ICM_UNION_FIND ? 1u : 0u;
     return PTICM_OK;
 }
 

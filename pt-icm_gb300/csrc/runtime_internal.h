@@ -82,6 +82,8 @@ constexpr uint32_t kSmemLimit = 232448 - 1024;   // 227 KB opt-in per block, les
 int choose_config(const HostProblem& P, const pticm_opts& o, bool replay, InstanceDesc& D, LaunchConfig& cfg,
                   std::string& msg);
 int engine_flags(const HostProblem& P, const pticm_opts& o);
+// Whether the union-find cluster search of a problem unites along every edge.
+bool icm_all_edges(const HostProblem& P);
 // Schedule of a launch that holds one instance: block b runs rank b.
 void single_instance_schedule(int group, std::vector<int32_t>& sched_off, std::vector<int32_t>& sched);
 // Per-instance engine choices of a configured instance: cluster search and

@@ -103,6 +103,7 @@ def lib():
         "pticm_icm_pairs": [P, P, u32, C.c_int],
         "pticm_get_exchange_order": [P, P],
         "pticm_get_layout": [P, C.POINTER(Layout)],
+        "pticm_get_paths": [P, P, P],
         "pticm_smem_copy_rate": [C.c_int, P],
         "pticm_set_wait_limit": [P, u64, u32],
         "pticm_philox_probe": [P, P, P, C.c_int],
@@ -375,6 +376,13 @@ class Context:
         out = Layout()
         _check(lib().pticm_get_layout(self._h, C.byref(out)))
         return out
+
+    def paths(self):
+        """Threads that gather one site's field (0: stored fields), and whether
+        the cluster search unites along every edge (else it samples links)."""
+        lanes, every = C.c_uint32(), C.c_uint32()
+        _check(lib().pticm_get_paths(self._h, C.byref(lanes), C.byref(every)))
+        return lanes.value, bool(every.value)
 
     def exchange_order(self):
         """The pair order of the reference-order exchange (nt-1 entries)."""
