@@ -470,7 +470,31 @@ void single_instance_schedule(int group, std::vector<int32_t>& sched_off, std::v
 // degree 6: 1.07 times slower; degree 30: 1.09 times faster; from degree 34 or
 // so the hot replicas' pushes are the critical path).  Lists in device memory
 // are gathered only for few neighbours (N=4541, degree 38: 1.13 times slower).
+//
+// Both costs are those of the mean list.  A class ends with its longest list,
+// which stored fields do not read: what uneven degrees cost a gathered sweep
+// grows with the longest list of each class, summed over the classes (degree
+// 8 on 1000 sites and one list of 100: gathered 17.2 against 17.3 us a step, of
+// 200: 18.2 against 17.5, of 400 18.9 against 17.6; eight of 200: 21.3 against
+// 17.6; a 44 x 44 lattice with one list of 200: 22.9 against 23.2, of 900: 26.0
+// against 18.8).  So gathered only while that sum is at most kChainBase and
+// kChainFew times that of mean lists; kChainMany times where the hot replicas'
+// pushes are the critical path (no ICM: degree 8, one list of 200 9.2 against
+// 9.6, of 400 10.0 against 9.5; degree 6 on 2000 sites, of 400 12.4 against
+// 11.3; degree 20 on 1500 sites, eight of 200: 16.7 against 16.9).
 constexpr double kGatherUpTo = 8.5, kGatherFrom = 34.0;
+constexpr double kChainBase = 120.0, kChainFew = 2.0, kChainMany = 4.0;
+
+// Sum over the colour classes of the longest neighbour list.
+static int64_t class_chain(const HostProblem& P) {
+    int64_t sum = 0;
+    for (int k = 0; k < P.ncolors; k++) {
+        int32_t longest = 0;
+        for (int i = P.color_off[k]; i < P.color_off[k + 1]; i++) longest = std::max(longest, P.drow[i + 1] - P.drow[i]);
+        sum += longest;
+    }
+    return sum;
+}
 
 // Threads per site: G threads share a list of `pieces` 16-byte pieces, a class
 // of S sites takes ceil(S G / threads) portions; a portion costs about 250
@@ -527,8 +551,9 @@ bool icm_all_edges(const HostProblem& P) {
 
 void finish_desc(InstanceDesc& D, const HostProblem& P, const pticm_opts& o, const LaunchConfig& cfg) {
     const double degree = (double)P.dadj.size() / (double)std::max<int64_t>(P.n, 1);
-    const bool gather = cfg.narrow && (degree <= kGatherUpTo || cfg.field_gather ||
-                                       (cfg.plan.stage_adj && (D.nc == 0 || degree >= kGatherFrom)));
+    const bool few = degree <= kGatherUpTo, many = cfg.plan.stage_adj && (D.nc == 0 || degree >= kGatherFrom);
+    const double chain = kChainBase + (few && D.nc > 0 ? kChainFew : kChainMany) * P.ncolors * degree;
+    const bool gather = cfg.narrow && (cfg.field_gather || ((few || many) && (double)class_chain(P) <= chain));
     D.lanes = gather ? gather_lanes(P, cfg.threads) : 0;
     D.icm_algo = engine_flags(P, o) & ENGINE_ICM_MASK;
     D.all_edges = icm_all_edges(P) ? 1 : 0;

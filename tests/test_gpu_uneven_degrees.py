@@ -95,3 +95,44 @@ def test_cluster_search_of_uneven_graphs(name):
         out.append(ctx.replicas())
     for a, b in zip(*out):
         assert np.array_equal(a, b)
+
+
+def _with_hubs(graph, count, length):
+    """`count` sites of a graph with `length` more neighbours each."""
+    n, e = graph
+    rng = np.random.default_rng(length)
+    more = [np.stack([np.full(length, k), rng.choice(np.arange(count, n), length, replace=False)], 1) for k in range(count)]
+    return n, np.unique(np.sort(np.concatenate([e] + more), 1), axis=0)
+
+
+FIELDS = {
+    "lattice": (_lattice(20), True, True),
+    "lattice_hub": (_hubs(20, 1, 180), False, False),
+    "lattice_short_hub": (_hubs(20, 1, 40), True, True),
+    "degree_8": (_random(1000, 4000), True, True),
+    "degree_8_hub": (_with_hubs(_random(1000, 4000), 1, 600), False, False),
+    "degree_8_hubs": (_with_hubs(_random(1000, 3000), 4, 200), False, False),
+    "degree_20": (_random(1500, 15000), False, True),
+    "degree_20_hub": (_with_hubs(_random(1500, 15000), 1, 1400), False, False),
+    "degree_40_hub": (_with_hubs(_random(1000, 20000), 1, 300), True, True),
+}
+
+
+@pytest.mark.parametrize("icm", [True, False])
+@pytest.mark.parametrize("name", list(FIELDS))
+def test_fields_of_uneven_graphs(name, icm):
+    graph, with_icm, without = FIELDS[name]
+    p, ctx = _context(graph, icm=icm)
+    assert (ctx.paths()[0] > 0) == (with_icm if icm else without)
+    ctx.run(25)
+    assert ctx.verify() == 0
+    s, E, _, _ = ctx.replicas()
+    assert np.array_equal(p.evaluate(s)[0].astype(np.int64), E)
+
+
+@pytest.mark.parametrize("n,deg", [(60, 14), (300, 20), (1000, 12), (2000, 20)])
+def test_between_the_degree_lines_the_two_sweeps_differ(n, deg):
+    """Graphs of these sizes store fields with ICM and gather without it."""
+    graph = _random(n, n * deg // 2)
+    assert _context(graph, icm=True)[1].paths()[0] == 0
+    assert _context(graph, icm=False)[1].paths()[0] > 0
