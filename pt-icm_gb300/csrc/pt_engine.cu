@@ -951,18 +951,34 @@ __device__ __forceinline__ int icm_pair(const EngineArgs& A, const BlockCtx& B, 
                 if (BLOCK) {
                     // the edges of S: one warp per site and one lane per
                     // neighbour (the unions of a site side by side) when
-                    // that takes fewer rounds than one thread per site
+                    // that takes fewer rounds than one thread per site; a
+                    // list far above the mean always by its warp (44 x 44
+                    // lattice and eight sites with 64 neighbours: step 46.2
+                    // -> 28.5 us)
                     const int ns0 = min(*(volatile int*)(team.ctl + TC_S), llen);
-                    const int nw = team.ts >> 5;
-                    const bool by_warp = (ns0 + nw - 1) / nw < (D.nnz + n - 1) / n;
+                    const int nw = team.ts >> 5, lane = team.tr & 31;
+                    const int mean = (D.nnz + n - 1) / n, long_list = max(16, 3 * mean);
+                    const bool by_warp = (ns0 + nw - 1) / nw < mean;
                     const int t0 = by_warp ? team.tr >> 5 : team.tr, dt = by_warp ? nw : team.ts;
-                    const int a0 = by_warp ? team.tr & 31 : 0, da = by_warp ? 32 : 1;
-                    for (int t = t0; t < ns0; t += dt) {
-                        const int u = lst[sbase + t];
-                        const int e1 = brow[u + 1];
-                        for (int a = brow[u] + a0; a < e1; a += da) {
+                    auto unite_list = [&](int u, int a, int e1, int da) {
+                        for (; a < e1; a += da) {
                             const int v = (int)(badj[a] >> 8);
                             if (d[v]) ok &= uf_unite(lab, u, v);
+                        }
+                    };
+                    for (int t = t0; t - (by_warp ? 0 : lane) < ns0; t += dt) {
+                        int u = 0, a = 0, e1 = 0;
+                        if (t < ns0) {
+                            u = lst[sbase + t];
+                            a = brow[u];
+                            e1 = brow[u + 1];
+                        }
+                        unsigned wide = by_warp ? 1u : __ballot_sync(0xffffffffu, e1 - a > long_list);
+                        if (!by_warp && e1 - a <= long_list) unite_list(u, a, e1, 1);
+                        for (; wide; wide &= wide - 1) {
+                            const int src = __ffs(wide) - 1;
+                            unite_list(__shfl_sync(0xffffffffu, u, src), __shfl_sync(0xffffffffu, a, src) + lane,
+                                       __shfl_sync(0xffffffffu, e1, src), 32);
                         }
                     }
                     team.sync();

@@ -71,6 +71,8 @@ GRAPHS = {
     "attached_2": (_attached(400, 2), False),
     "attached_2_large": (_attached(2400, 2), False),
     "star": (_star(700), False),
+    "long_lists_outside": (_hubs(44, 8, 64), False),   # united by a warp each
+    "lists_around_the_warp_line": (_hubs(44, 12, 17), False),
     "ring": (_ring(2501), True),
     "random_1000": (_random(1000, 1250), True),
     "random_2000": (_random(2000, 2500), False),
