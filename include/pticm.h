@@ -479,6 +479,15 @@ PTICM_API int pticm_batch_get_energy_histograms(pticm_batch* b, uint32_t inst, u
 /* The multihistogram ln g of every instance in one device launch (kept for
  * pticm_batch_logdos until the next run). */
 PTICM_API int pticm_batch_compute_logdos(pticm_batch* b, double estep);
+
+/* The same with a bound on the device memory that the solve holds beside its
+ * inputs and results.  Instances whose matrix of bins x temperatures does not
+ * fit shared memory share slots of the largest one's size: as many as the GPU
+ * works on at once and `max_workspace` bytes hold, but one.  0 takes none and
+ * solves them in the log domain (slower, the same fixed point).  The call above
+ * takes at most 4 GiB, and less where memory is short.  `used` (may be NULL)
+ * receives the bytes taken. */
+PTICM_API int pticm_batch_compute_logdos_bounded(pticm_batch* b, double estep, uint64_t max_workspace, uint64_t* used);
 /* The FP64 multihistogram ln g of one instance from its histograms
  * (temperatures merged over chains; make_histogram and get_partition_iterate,
  * src/cae_estimator.cc:45-69,228-253).  Bin k is energy min_emin + k*estep. */

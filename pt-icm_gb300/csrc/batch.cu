@@ -848,6 +848,10 @@ int pticm_batch_get_energy_histograms(pticm_batch* b, uint32_t inst, uint32_t* h
 }
 
 int pticm_batch_compute_logdos(pticm_batch* b, double estep) {
+    return pticm_batch_compute_logdos_bounded(b, estep, kMhistWorkspace, nullptr);
+}
+
+int pticm_batch_compute_logdos_bounded(pticm_batch* b, double estep, uint64_t max_workspace, uint64_t* used) {
     if (!b || !(estep > 0)) return bfail(PTICM_ERR_INVALID, "invalid arguments");
     if (!b->hist_on) return bfail(PTICM_ERR_INVALID, "energy histograms are not enabled");
     BCK(cudaStreamSynchronize(b->stream));
@@ -879,7 +883,10 @@ int pticm_batch_compute_logdos(pticm_batch* b, double estep) {
         if (rc[i]) return bfail(rc[i], "instance " + std::to_string(i) + ": pilot histograms unusable");
     std::vector<const MhInput*> ptrs;
     for (auto& x : in) ptrs.push_back(&x);
-    if (int r = mhist_dos_multi(ptrs, b->dos)) return r;
+    MhWorkspace ws;
+    ws.most = (size_t)max_workspace;
+    if (int r = mhist_dos_multi(ptrs, b->dos, &ws)) return r;
+    if (used) *used = ws.used;
     b->dos_estep = estep;
     return PTICM_OK;
 }

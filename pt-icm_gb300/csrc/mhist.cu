@@ -142,13 +142,18 @@ __device__ bool mh_converged(const double* zold, const double* znew, int nt) {
     return !(metric > 1e-7);
 }
 
+// MANY: the clusters take the jobs in turn (else one job each).
+template <bool MANY>
 __global__ void __launch_bounds__(kMhThreads, 1)
-mh_solve_kernel(const MhJob* jobs, const uint32_t* hist, const uint64_t* hoff, const uint64_t* hlen, const double* emin,
-                const double* beta, double* logdos, double* logc, float* ldf, double* logZ, unsigned long long* iters,
-                long long max_iters, uint8_t* work, const long long* work_off, size_t smem_bytes) {
+mh_solve_kernel(int njobs, const MhJob* jobs, const uint32_t* hist, const uint64_t* hoff, const uint64_t* hlen,
+                const double* emin, const double* beta, double* logdos, double* logc, float* ldf, double* logZ,
+                unsigned long long* iters, long long max_iters, uint8_t* work, size_t slot, int* taken, size_t smem_bytes) {
     cg::cluster_group cluster = cg::this_cluster();
     const int cs = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
-    const int job = (int)blockIdx.x / cs;
+    const int mine = (int)blockIdx.x / cs, clusters = (int)gridDim.x / cs;
+    __shared__ int s_job;
+    // the cluster's first job, then those that no cluster has taken
+    for (int job = mine; !MANY || job < njobs;) {
     const MhJob J = jobs[job];
     const int nt = J.nt, tid = threadIdx.x, T = blockDim.x, p = mh_pitch(nt);
     const long long per = (J.nbins + cs - 1) / cs;
@@ -167,10 +172,11 @@ mh_solve_kernel(const MhJob* jobs, const uint32_t* hist, const uint64_t* hoff, c
     float* const sAf = reinterpret_cast<float*>(inbox + 2 * cs * nt);
     float* const sBf = sAf + nt;
     const size_t fixed = mh_fixed_bytes(nt, cs);
-    // the slice in shared memory when it fits, else in device memory (L2)
-    uint8_t* const slice = fixed + mh_slice_bytes(per, nt) <= smem_bytes
-                               ? mh_sm + fixed
-                               : work + work_off[job] + (size_t)rank * mh_slice_bytes(per, nt);
+    // the slice in shared memory when it fits, else in the cluster's slot of
+    // device memory (L2); without one every iteration is made in the log domain
+    const bool in_smem = fixed + mh_slice_bytes(per, nt) <= smem_bytes, matrix = in_smem || work != nullptr;
+    uint8_t* const slice = in_smem ? mh_sm + fixed
+                           : matrix ? work + (size_t)mine * slot + (size_t)rank * mh_slice_bytes(per, nt) : nullptr;
     double* const K = reinterpret_cast<double*>(slice);
     double* const c = K + (size_t)per * p;
     double* const g = c + per;
@@ -203,7 +209,7 @@ mh_solve_kernel(const MhJob* jobs, const uint32_t* hist, const uint64_t* hoff, c
             if (idx >= (double)hl[j]) continue;
             count += hist[ho[j] + (uint64_t)idx];
         }
-        c[r] = (double)count;
+        if (matrix) c[r] = (double)count;
         lc[i] = count ? log((double)count) : -DBL_MAX;
     }
     __threadfence();
@@ -230,7 +236,7 @@ mh_solve_kernel(const MhJob* jobs, const uint32_t* hist, const uint64_t* hoff, c
                     far = fmaxf(far, dz);
                 }
                 s_flag[0] = mh_converged(sZ, sNew, nt);
-                s_flag[1] = finite && far < kFarNats ? NEXT_REF : NEXT_LOG;
+                s_flag[1] = matrix && finite && far < kFarNats ? NEXT_REF : NEXT_LOG;
                 for (int j = 0; j < nt; j++) sZ[j] = sNew[j];
             }
             cluster.sync();   // the inbox is read before anyone writes it again
@@ -412,6 +418,15 @@ mh_solve_kernel(const MhJob* jobs, const uint32_t* hist, const uint64_t* hoff, c
         for (int j = tid; j < nt; j += T) logZ[J.row0 + j] = sZ[j];
         if (tid == 0) iters[job] = (unsigned long long)it;
     }
+    if (!MANY) break;
+    if (rank == 0 && tid == 0) {
+        const int next = clusters + atomicAdd(taken, 1);
+        for (int q = 0; q < cs; q++) *cluster.map_shared_rank(&s_job, q) = next;
+    }
+    cluster.sync();
+    job = s_job;
+    cluster.sync();   // (read before it is written again)
+    }
     cluster.sync();   // no CTA leaves while another may still write to its shared memory
 }
 
@@ -428,8 +443,8 @@ static int mh_cluster_size(const std::vector<MhJob>& jobs, int max_nt, int sms) 
     return cs;
 }
 
-static void mhist_config(int njobs, int cs, cudaStream_t st, cudaLaunchConfig_t& cfg, cudaLaunchAttribute* attr) {
-    cfg.gridDim = dim3((unsigned)njobs * (unsigned)cs);
+static void mhist_config(int clusters, int cs, cudaStream_t st, cudaLaunchConfig_t& cfg, cudaLaunchAttribute* attr) {
+    cfg.gridDim = dim3((unsigned)clusters * (unsigned)cs);
     cfg.blockDim = dim3(kMhThreads);
     cfg.dynamicSmemBytes = kMhSmem;
     cfg.stream = st;
@@ -441,46 +456,64 @@ static void mhist_config(int njobs, int cs, cudaStream_t st, cudaLaunchConfig_t&
     cfg.numAttrs = 1;
 }
 
-// The launch of a solve: CTAs per instance and, for the slices that do not fit
-// shared memory, the bytes of device memory and every job's offset in it.
-cudaError_t mhist_plan(const std::vector<MhJob>& jobs, int max_nt, int& cs, size_t& bytes, std::vector<long long>& off) {
+template <class Kernel>
+static cudaError_t mhist_allow(Kernel kernel) {
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMhSmem);
+    return e != cudaSuccess ? e : cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+}
+
+// The launch of a solve: CTAs per instance, clusters and, for slices that do
+// not fit shared memory, a slot of device memory for each cluster (0: all fit).
+// A slot holds the largest such instance and its cluster's next instances use
+// it again, so a launch with slots has only as many clusters as the GPU runs at
+// once and `most` bytes of slots (but one slot); the clusters take the instances
+// in turn.  (A matrix per instance, 8 bytes a bin and temperature each, grew with
+// the number of instances: 1000 of 20000 bins and 128 temperatures 21 GB.)
+cudaError_t mhist_plan(const std::vector<MhJob>& jobs, int max_nt, size_t most, int& cs, int& clusters, size_t& slot) {
     // (more temperatures than a launch has ever taken)
     if ((size_t)max_nt * (4 * sizeof(double) + 2 * sizeof(float)) > 48 * 1024) return cudaErrorInvalidValue;
     int dev = 0, sms = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(mh_solve_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMhSmem);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(mh_solve_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if (e == cudaSuccess) e = mhist_allow(mh_solve_kernel<false>);
     if (e != cudaSuccess) return e;
     cs = mh_cluster_size(jobs, max_nt, sms);
+    int resident = sms / cs;
     while (cs > 8) {   // (above the portable size: when the GPU can place one)
         cudaLaunchConfig_t cfg = {};
         cudaLaunchAttribute attr[1];
         mhist_config((int)jobs.size(), cs, nullptr, cfg, attr);
-        int clusters = 0;
-        if (cudaOccupancyMaxActiveClusters(&clusters, mh_solve_kernel, &cfg) == cudaSuccess && clusters > 0) break;
+        int placed = 0;
+        if (cudaOccupancyMaxActiveClusters(&placed, mh_solve_kernel<false>, &cfg) == cudaSuccess && placed > 0) {
+            resident = placed;
+            break;
+        }
         cudaGetLastError();
         cs /= 2;
+        resident = sms / cs;
     }
-    off.clear();
-    bytes = 0;
+    clusters = (int)jobs.size();
+    slot = 0;
     for (const MhJob& J : jobs) {
-        off.push_back((long long)bytes);
         const size_t slice = mh_slice_bytes((J.nbins + cs - 1) / cs, J.nt);
-        if (mh_fixed_bytes(J.nt, cs) + slice > kMhSmem) bytes = (bytes + cs * slice + 127) & ~size_t(127);
+        if (mh_fixed_bytes(J.nt, cs) + slice > kMhSmem) slot = std::max(slot, (cs * slice + 127) & ~size_t(127));
     }
+    if (slot) clusters = std::min<int>(std::min(clusters, resident), (int)std::max<size_t>(1, std::min(most / slot, (size_t)clusters)));
     return cudaSuccess;
 }
 
-cudaError_t mhist_solve(int njobs, int cs, const MhJob* jobs, const uint32_t* hist, const uint64_t* hoff,
+cudaError_t mhist_solve(int njobs, int cs, int clusters, const MhJob* jobs, const uint32_t* hist, const uint64_t* hoff,
                         const uint64_t* hlen, const double* emin, const double* beta, double* logdos, double* logc,
                         float* ldf, double* logZ, unsigned long long* iters, long long max_iters, uint8_t* work,
-                        const long long* work_off, cudaStream_t st) {
+                        size_t slot, int* taken, cudaStream_t st) {
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[1];
-    mhist_config(njobs, cs, st, cfg, attr);
-    return cudaLaunchKernelEx(&cfg, mh_solve_kernel, jobs, hist, hoff, hlen, emin, beta, logdos, logc, ldf, logZ, iters,
-                              max_iters, work, work_off, kMhSmem);
+    mhist_config(clusters, cs, st, cfg, attr);
+    const auto kernel = clusters < njobs ? mh_solve_kernel<true> : mh_solve_kernel<false>;
+    const cudaError_t e = mhist_allow(kernel);
+    if (e != cudaSuccess) return e;
+    return cudaLaunchKernelEx(&cfg, kernel, njobs, jobs, hist, hoff, hlen, emin, beta, logdos, logc, ldf, logZ,
+                              iters, max_iters, work, slot, taken, kMhSmem);
 }
 
 }  // namespace pticm

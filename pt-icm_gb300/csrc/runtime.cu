@@ -744,11 +744,11 @@ int reset_run_state(pticm_ctx* c) {
 }  // namespace
 
 namespace pticm {
-cudaError_t mhist_plan(const std::vector<MhJob>& jobs, int max_nt, int& cs, size_t& bytes, std::vector<long long>& off);
-cudaError_t mhist_solve(int njobs, int cs, const MhJob* jobs, const uint32_t* hist, const uint64_t* hoff,
+cudaError_t mhist_plan(const std::vector<MhJob>& jobs, int max_nt, size_t most, int& cs, int& clusters, size_t& slot);
+cudaError_t mhist_solve(int njobs, int cs, int clusters, const MhJob* jobs, const uint32_t* hist, const uint64_t* hoff,
                         const uint64_t* hlen, const double* emin, const double* beta, double* logdos, double* logc,
                         float* ldf, double* logZ, unsigned long long* iters, long long max_iters, uint8_t* work,
-                        const long long* work_off, cudaStream_t st);
+                        size_t slot, int* taken, cudaStream_t st);
 }  // namespace pticm
 
 namespace pticm {
@@ -756,7 +756,7 @@ namespace pticm {
 // The multihistogram fixed point on the GPU (src/cae_estimator.cc:228-253)
 // for any number of histogram sets in one launch (mhist_solve): iterate
 // until sum_j ((lnZ_j - lnZ'_j)/lnZ'_j)^2 <= 1e-7, as the reference does.
-int mhist_dos_multi(const std::vector<const MhInput*>& in, std::vector<MhOutput>& out) {
+int mhist_dos_multi(const std::vector<const MhInput*>& in, std::vector<MhOutput>& out, MhWorkspace* ws) {
     const size_t K = in.size();
     out.assign(K, MhOutput{});
     std::vector<MhJob> jobs;
@@ -809,13 +809,21 @@ int mhist_dos_multi(const std::vector<const MhInput*>& in, std::vector<MhOutput>
     DArr<double> d_emin, d_beta, d_logZ, d_dos, d_logc;
     DArr<float> d_ldf;
     DArr<uint8_t> d_work;
-    DArr<long long> d_work_off;
-    std::vector<long long> work_off;
-    int cs = 1;
-    size_t work_bytes = 0;
-    CK(mhist_plan(jobs, max_nt, cs, work_bytes, work_off));
-    CK(d_work.alloc(work_bytes));
-    CK(d_work_off.upload(work_off));
+    DArr<int> d_taken;
+    int cs = 1, clusters = 1;
+    size_t slot = 0;
+    CK(mhist_plan(jobs, max_nt, ws ? ws->most : kMhistWorkspace, cs, clusters, slot));
+    if (slot && !(ws && ws->most == 0)) {
+        // (fewer slots where memory is short; without any, the log domain)
+        while (d_work.reserve((size_t)clusters * slot) != cudaSuccess) {
+            cudaGetLastError();
+            if (clusters == 1) break;
+            clusters /= 2;
+        }
+    }
+    if (slot && !d_work.p) clusters = (int)jobs.size();
+    if (ws) ws->used = d_work.n;
+    CK(d_taken.alloc(1));
     CK(d_jobs.upload(jobs));
     CK(d_hist.upload(hist, 1));
     CK(d_off.upload(hoff));
@@ -827,8 +835,8 @@ int mhist_dos_multi(const std::vector<const MhInput*>& in, std::vector<MhOutput>
     CK(d_logc.alloc((size_t)bins));
     CK(d_ldf.alloc((size_t)bins));
     CK(d_it.alloc(jobs.size()));
-    CK(mhist_solve((int)jobs.size(), cs, d_jobs.p, d_hist.p, d_off.p, d_len.p, d_emin.p, d_beta.p, d_dos.p,
-                   d_logc.p, d_ldf.p, d_logZ.p, d_it.p, kMhistMaxIters, d_work.p, d_work_off.p, nullptr));
+    CK(mhist_solve((int)jobs.size(), cs, clusters, d_jobs.p, d_hist.p, d_off.p, d_len.p, d_emin.p, d_beta.p, d_dos.p,
+                   d_logc.p, d_ldf.p, d_logZ.p, d_it.p, kMhistMaxIters, d_work.p, slot, d_taken.p, nullptr));
     CK(cudaDeviceSynchronize());
     std::vector<double> dos, z;
     std::vector<unsigned long long> it;

@@ -108,7 +108,14 @@ struct MhOutput {
     uint64_t iters = 0;
 };
 constexpr long long kMhistMaxIters = 300000;
-int mhist_dos_multi(const std::vector<const MhInput*>& in, std::vector<MhOutput>& out);
+// Device memory for the matrices of a solve whose instances do not fit shared
+// memory: at most `most` bytes (but one instance's), or 0 for none; `used` is
+// what it took.
+struct MhWorkspace {
+    size_t most = 0, used = 0;
+};
+constexpr size_t kMhistWorkspace = (size_t)4 << 30;
+int mhist_dos_multi(const std::vector<const MhInput*>& in, std::vector<MhOutput>& out, MhWorkspace* ws = nullptr);
 int compact_slot_hist(const unsigned* rows, int nt, int chains, long long nbins, long long lo, const double* hb,
                       double estep, MhInput& I);
 int mhist_dos_impl(const uint32_t* hist, const uint64_t* hoff, const uint64_t* hlen, uint32_t nt,

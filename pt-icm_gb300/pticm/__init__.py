@@ -132,6 +132,7 @@ def lib():
         "pticm_batch_get_energy_histograms": [P, u32, P, P, P],
         "pticm_batch_logdos": [P, u32, dbl, P, u64, P, P, P],
         "pticm_batch_compute_logdos": [P, dbl],
+        "pticm_batch_compute_logdos_bounded": [P, dbl, u64, P],
         "pticm_mlp_create": [u64, u32, C.POINTER(P)],
         "pticm_mlp_get_params": [P, P],
         "pticm_mlp_set_params": [P, P],
@@ -610,9 +611,14 @@ class Batch:
         _check(lib().pticm_batch_get_energy_histograms(self._h, inst, _p(h), C.byref(lo), C.byref(nb)))
         return h, lo.value + 2 * np.arange(nb.value)
 
-    def compute_logdos(self, estep=2.0):
-        """ln g of every instance in one device launch (cached for logdos)."""
-        _check(lib().pticm_batch_compute_logdos(self._h, estep))
+    def compute_logdos(self, estep=2.0, max_workspace=None):
+        """ln g of every instance in one device launch (cached for logdos).
+        Returns the device bytes held for matrices that do not fit shared
+        memory, at most max_workspace (default 4 GiB; 0: the log domain)."""
+        used = C.c_uint64()
+        most = 4 << 30 if max_workspace is None else max_workspace
+        _check(lib().pticm_batch_compute_logdos_bounded(self._h, estep, most, C.byref(used)))
+        return used.value
 
     def logdos(self, inst, estep=2.0):
         hb = C.c_uint64()
