@@ -337,12 +337,14 @@ int pticm_mlp_train(pticm_mlp* m, const float* x, const float* y, uint64_t n, ui
         uint32_t* hring = nullptr;   // pinned host
         float* losses = nullptr;     // device, one per step
         cudaEvent_t copied[2] = {nullptr, nullptr};
+        cudaEvent_t ready = nullptr;
         ~Res() {
             if (st) cudaStreamSynchronize(st);
             if (exec) cudaGraphExecDestroy(exec);
             if (graph) cudaGraphDestroy(graph);
             for (cudaEvent_t e : copied)
                 if (e) cudaEventDestroy(e);
+            if (ready) cudaEventDestroy(ready);
             if (st) cudaStreamDestroy(st);
             cudaFree(ring);
             cudaFree(losses);
@@ -354,6 +356,11 @@ int pticm_mlp_train(pticm_mlp* m, const float* x, const float* y, uint64_t n, ui
     MLP_CK(cudaMalloc(&r.losses, (size_t)steps * 4));
     MLP_CK(cudaMallocHost(&r.hring, 2 * half * 4));
     for (cudaEvent_t& e : r.copied) MLP_CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    MLP_CK(cudaEventCreateWithFlags(&r.ready, cudaEventDisableTiming));
+    // the dataset's copies and the weights' images were issued on the default
+    // stream, which r.st does not wait for by itself
+    MLP_CK(cudaEventRecord(r.ready, nullptr));
+    MLP_CK(cudaStreamWaitEvent(r.st, r.ready, 0));
     MLP_CK(cudaMemsetAsync(m->a.status, 0, sizeof(DevStatus), r.st));
     MLP_CK(cudaMemsetAsync(m->a.abort_flag, 0, sizeof(int), r.st));
     MLP_CK(cudaMemsetAsync(m->ctr, 0, sizeof(long long), r.st));   // this call's iteration counter
