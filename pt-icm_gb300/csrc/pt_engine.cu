@@ -960,12 +960,6 @@ __device__ __forceinline__ int icm_pair(const EngineArgs& A, const BlockCtx& B, 
                     const int mean = (D.nnz + n - 1) / n, long_list = max(16, 3 * mean);
                     const bool by_warp = (ns0 + nw - 1) / nw < mean;
                     const int t0 = by_warp ? team.tr >> 5 : team.tr, dt = by_warp ? nw : team.ts;
-                    auto unite_list = [&](int u, int a, int e1, int da) {
-                        for (; a < e1; a += da) {
-                            const int v = (int)(badj[a] >> 8);
-                            if (d[v]) ok &= uf_unite(lab, u, v);
-                        }
-                    };
                     for (int t = t0; t - (by_warp ? 0 : lane) < ns0; t += dt) {
                         int u = 0, a = 0, e1 = 0;
                         if (t < ns0) {
@@ -973,12 +967,22 @@ __device__ __forceinline__ int icm_pair(const EngineArgs& A, const BlockCtx& B, 
                             a = brow[u];
                             e1 = brow[u + 1];
                         }
+                        // a thread's own list, then the warp's long ones
                         unsigned wide = by_warp ? 1u : __ballot_sync(0xffffffffu, e1 - a > long_list);
-                        if (!by_warp && e1 - a <= long_list) unite_list(u, a, e1, 1);
-                        for (; wide; wide &= wide - 1) {
-                            const int src = __ffs(wide) - 1;
-                            unite_list(__shfl_sync(0xffffffffu, u, src), __shfl_sync(0xffffffffu, a, src) + lane,
-                                       __shfl_sync(0xffffffffu, e1, src), 32);
+                        int x = u, b = e1 - a > long_list ? e1 : a, be = e1, db = 1;
+                        for (bool own = !by_warp; own || wide; own = false) {
+                            if (!own) {
+                                const int src = __ffs(wide) - 1;
+                                x = __shfl_sync(0xffffffffu, u, src);
+                                b = __shfl_sync(0xffffffffu, a, src) + lane;
+                                be = __shfl_sync(0xffffffffu, e1, src);
+                                db = 32;
+                                wide &= wide - 1;
+                            }
+                            for (; b < be; b += db) {
+                                const int v = (int)(badj[b] >> 8);
+                                if (d[v]) ok &= uf_unite(lab, x, v);
+                            }
                         }
                     }
                     team.sync();
