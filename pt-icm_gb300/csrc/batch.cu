@@ -268,6 +268,7 @@ int configure_batch(pticm_batch* b) {
     BCK(b->d_desc.upload(b->desc));
     BCK(b->d_sched_off.upload(b->sched_off));
     BCK(b->d_sched.upload(b->sched));
+    BCK(default_stream_done());
     return PTICM_OK;
 }
 
@@ -395,7 +396,7 @@ struct Snapshot {
 template <typename T>
 cudaError_t dcopy(DArr<T>& dst, const DArr<T>& src, cudaStream_t st) {
     if (dst.n != src.n) {
-        cudaError_t e = dst.alloc(src.n);
+        cudaError_t e = dst.reserve(src.n);
         if (e != cudaSuccess) return e;
     }
     if (!src.n) return cudaSuccess;
@@ -520,6 +521,7 @@ int pticm_batch_create(const pticm_problem* const* problems, uint32_t count, con
     BCK(b->d_abort.alloc(1));
     BCK(b->d_status.alloc(1));
     BCK(b->d_mismatch.alloc(1));
+    BCK(default_stream_done());
     // smallest group per instance: replicas of a block fit shared memory
     // (unstaged, one ICM team) on their own
     b->gmin.assign(count, 0);
@@ -568,6 +570,7 @@ int pticm_batch_set_ladders(pticm_batch* b, const double* beta, uint32_t nt, int
     }
     BCK(b->d_beta.upload(b->beta));
     BCK(b->d_thr.upload(thr_all, 4));
+    BCK(default_stream_done());
     b->ladder_set = true;
     return PTICM_OK;
 }
@@ -642,6 +645,7 @@ int pticm_batch_autotune(pticm_batch* b, uint32_t trial_steps) {
         }
         DArr<unsigned long long> job_ns;
         BCK(job_ns.alloc(b->sched.size() / 2));
+        BCK(default_stream_done());
         // a two-step launch sizes the trial so that it stays near the launch target
         float ms = 0.f;
         if (int rc = batch_launch(b, b->steps_done, 2, PHASE_SWEEP | PHASE_EXCHANGE | PHASE_ICM, nullptr, &ms))
@@ -828,6 +832,7 @@ int pticm_batch_enable_energy_histograms(pticm_batch* b, uint64_t from_step) {
     }
     if ((uint64_t)off > (1ull << 34)) return bfail(PTICM_ERR_UNSUPPORTED, "energy histograms of the batch exceed 64 GB");
     BCK(b->d_hist.alloc((size_t)off));
+    BCK(default_stream_done());
     b->hist_from = from_step;
     b->hist_on = true;
     return PTICM_OK;

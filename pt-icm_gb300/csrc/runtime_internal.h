@@ -15,6 +15,11 @@ namespace pticm {
 
 constexpr long long kNoBest = std::numeric_limits<long long>::max();
 
+// The runtime's streams do not wait for the default stream, on which DArr
+// clears and fills its buffers (a clear, or a copy from pageable memory, may
+// return before it has landed): called before such buffers are used on them.
+inline cudaError_t default_stream_done() { return cudaStreamSynchronize(cudaStreamLegacy); }
+
 template <typename T>
 struct DArr {
     T* p = nullptr;
