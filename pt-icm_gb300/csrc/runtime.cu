@@ -78,6 +78,10 @@ struct pticm_problem {
     bool uploaded = false;
 };
 
+// Device memory that pticm_get_replicas holds for the reordered rows (but one
+// replica's).
+constexpr size_t kExportBytes = (size_t)64 << 20;
+
 struct pticm_ctx {
     HostProblem P;
     pticm_opts o{};
@@ -110,8 +114,8 @@ struct pticm_ctx {
     DArr<unsigned int> d_bar;
     DArr<int> d_abort;
     DArr<DevStatus> d_status;
-    DArr<uint8_t> d_states_in;  // states in the original site order (pticm_set_states, pticm_get_replicas)
-    DArr<int32_t> d_fields_out; // fields in the original site order (pticm_get_replicas)
+    DArr<uint8_t> d_states_in;  // caller states in the original site order (pticm_set_states)
+    DArr<uint8_t> d_export;     // fields and states of some replicas in the original site order (pticm_get_replicas)
     DArr<uint8_t> d_icm_pool;   // ICM scratch when the replicas live in device memory
     long long icm_stride = 0;
     DArr<unsigned long long> d_icm_pub;   // per pair what is flipped (large instances)
@@ -1425,15 +1429,20 @@ int pticm_get_replicas(pticm_ctx* c, uint8_t* states, int64_t* energy, int32_t* 
     CK(cudaStreamSynchronize(c->stream));
     const int n = (int)c->P.n, npad = c->desc.n_pad;
     if (states || fields) {
-        // into the original order on the device, then straight to the caller
-        const size_t sites = (size_t)c->R * (size_t)n;
-        DArr<int32_t>& d_f = c->d_fields_out;
-        if (states && c->d_states_in.n != sites) CK(c->d_states_in.reserve(sites));
-        if (fields && d_f.n != sites) CK(d_f.reserve(sites));
-        CK(launch_export(c->d_spins.p, c->d_fields.p, c->d_perm.p, states ? c->d_states_in.p : nullptr, fields ? d_f.p : nullptr, c->R, n, npad,
-                         c->stream));
-        if (states) CK(cudaMemcpyAsync(states, c->d_states_in.p, sites, cudaMemcpyDeviceToHost, c->stream));
-        if (fields) CK(cudaMemcpyAsync(fields, d_f.p, sites * sizeof(int32_t), cudaMemcpyDeviceToHost, c->stream));
+        // into the original order on the device, then straight to the caller,
+        // as many replicas at a time as fit the export buffer
+        const size_t fb = fields ? sizeof(int32_t) * (size_t)n : 0, sb = states ? (size_t)n : 0;
+        const int per = (int)std::min<size_t>((size_t)c->R, std::max<size_t>(1, kExportBytes / (fb + sb)));
+        if (c->d_export.n < (size_t)per * (fb + sb)) CK(c->d_export.reserve((size_t)per * (fb + sb)));
+        int32_t* const f = fields ? reinterpret_cast<int32_t*>(c->d_export.p) : nullptr;
+        uint8_t* const s = states ? c->d_export.p + (size_t)per * fb : nullptr;
+        for (int r0 = 0; r0 < c->R; r0 += per) {
+            const int cnt = std::min(per, c->R - r0);
+            const size_t from = (size_t)r0 * npad;
+            CK(launch_export(c->d_spins.p + from, c->d_fields.p + from, c->d_perm.p, s, f, cnt, n, npad, c->stream));
+            if (states) CK(cudaMemcpyAsync(states + (size_t)r0 * n, s, cnt * sb, cudaMemcpyDeviceToHost, c->stream));
+            if (fields) CK(cudaMemcpyAsync(fields + (size_t)r0 * n, f, cnt * fb, cudaMemcpyDeviceToHost, c->stream));
+        }
         CK(cudaStreamSynchronize(c->stream));
     }
     if (energy) {
