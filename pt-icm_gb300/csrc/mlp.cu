@@ -127,6 +127,9 @@ extern "C" int pticm_tc_gemm_bench(int M, int N, int K, int iters, double* ms_pe
 // ===================================================================== MLP
 namespace {
 
+// Rows of a prediction on the device at a time (128 MB with their results).
+constexpr uint64_t kPredictRows = (uint64_t)4 << 20;
+
 const size_t kWoff[MLP_LAYERS] = {kW1, kW2, kW3, kW4};
 const int kKin[MLP_LAYERS] = {MLP_K0, MLP_H, MLP_H, MLP_H};
 
@@ -404,16 +407,21 @@ int pticm_mlp_train(pticm_mlp* m, const float* x, const float* y, uint64_t n, ui
 int pticm_mlp_predict(pticm_mlp* m, const float* x, uint64_t n, float* y) {
     if (!m || !x || !y) return mlp_fail(PTICM_ERR_INVALID, "null argument");
     if (n == 0) return PTICM_OK;
-    if (int rc = mlp_upload_rows(m, x, n)) return rc;
-    if (int rc = mlp_reserve(&m->y, &m->cap_p, n, 1)) return rc;
-    MLP_CK(cudaMemsetAsync(m->a.status, 0, sizeof(DevStatus), nullptr));
-    MLP_CK(cudaMemsetAsync(m->a.abort_flag, 0, sizeof(int), nullptr));
-    MlpArgs A = m->a;
-    A.X = m->dX;
-    A.y = m->y;
-    A.n_valid = (long long)n;
-    MLP_CK(mlp_predict_rows(A, nullptr));
-    MLP_CK(cudaMemcpy(y, m->y, n * 4, cudaMemcpyDeviceToHost));
+    for (uint64_t r0 = 0; r0 < n; r0 += kPredictRows) {
+        const uint64_t rows = std::min(n - r0, kPredictRows);
+        if (int rc = mlp_upload_rows(m, x + r0 * MLP_IN, rows)) return rc;
+        if (int rc = mlp_reserve(&m->y, &m->cap_p, rows, 1)) return rc;
+        if (r0 == 0) {   // (behind the copy, which would wait for them)
+            MLP_CK(cudaMemsetAsync(m->a.status, 0, sizeof(DevStatus), nullptr));
+            MLP_CK(cudaMemsetAsync(m->a.abort_flag, 0, sizeof(int), nullptr));
+        }
+        MlpArgs A = m->a;
+        A.X = m->dX;
+        A.y = m->y;
+        A.n_valid = (long long)rows;
+        MLP_CK(mlp_predict_rows(A, nullptr));
+        MLP_CK(cudaMemcpy(y + r0, m->y, rows * 4, cudaMemcpyDeviceToHost));
+    }
     return mlp_check_status(m);
 }
 

@@ -28,3 +28,19 @@ def test_each_training_call_reads_its_own_rows_and_weights(rows):
         want, _ = fresh.gradients(X, y)
         # rows / 128 tile sums of 128 squares each, in another order: rows x 2^-24 relative at most
         assert abs(first - want) <= rows * 2.0 ** -24 * want, (k, first, want)
+
+
+def test_predictions_in_portions():
+    """More rows than one portion holds: each row's result is that of any other call, and device memory stays bounded."""
+    torch = pytest.importorskip("torch")
+    import pticm
+    net = pticm.MLP(seed=1, batch=256)
+    net.params = MO.init_like_device(3).astype(np.float32)
+    part, n = 4 << 20, (4 << 20) + 777
+    X = np.random.default_rng(0).standard_normal((n, MO.IN), dtype=np.float32)
+    small = net.predict(X[part - 100:])
+    before = torch.cuda.mem_get_info()[0]
+    y = net.predict(X)
+    assert before - torch.cuda.mem_get_info()[0] <= part * 32 + (8 << 20)   # (allocations come in 2 MB pieces)
+    assert np.array_equal(y[part - 100:], small)
+    assert np.array_equal(y[:1000], net.predict(X[:1000]))
