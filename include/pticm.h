@@ -582,6 +582,8 @@ PTICM_API const char* pticm_last_error(void);
 PTICM_API const char* pticm_version(void);
 /* Philox4x32-10 known-answer probe: out[4*i..] = philox(ctr[4*i..], key[2*i..]). */
 PTICM_API int pticm_philox_probe(const uint32_t* ctr, const uint32_t* key, uint32_t* out, int count);
+/* The surrogate network's branch-free division: q[i] = a[i] / b[i]. */
+PTICM_API int pticm_mlp_division_probe(const float* a, const float* b, float* q, int count);
 
 #ifdef __cplusplus
 }

@@ -425,4 +425,20 @@ int pticm_mlp_predict(pticm_mlp* m, const float* x, uint64_t n, float* y) {
     return mlp_check_status(m);
 }
 
+int pticm_mlp_division_probe(const float* a, const float* b, float* q, int count) {
+    if (!a || !b || !q || count <= 0) return mlp_fail(PTICM_ERR_INVALID, "invalid arguments");
+    int devices = 0;
+    if (cudaGetDeviceCount(&devices) != cudaSuccess || devices == 0)
+        return mlp_fail(PTICM_ERR_NODEVICE, "no CUDA device is available");
+    DArr<float> da, db, dq;
+    MLP_CK(da.reserve((size_t)count));
+    MLP_CK(db.reserve((size_t)count));
+    MLP_CK(dq.reserve((size_t)count));
+    MLP_CK(cudaMemcpy(da.p, a, (size_t)count * 4, cudaMemcpyHostToDevice));
+    MLP_CK(cudaMemcpy(db.p, b, (size_t)count * 4, cudaMemcpyHostToDevice));
+    MLP_CK(mlp_div(da.p, db.p, dq.p, count, nullptr));
+    MLP_CK(cudaMemcpy(q, dq.p, (size_t)count * 4, cudaMemcpyDeviceToHost));
+    return PTICM_OK;
+}
+
 }  // extern "C"

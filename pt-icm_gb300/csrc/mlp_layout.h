@@ -71,6 +71,7 @@ struct MlpArgs {
 };
 
 cudaError_t mlp_images(const float* P, uint8_t* const* Wi, uint8_t* const* WTi, cudaStream_t st);
+cudaError_t mlp_div(const float* a, const float* b, float* q, long long count, cudaStream_t st);
 cudaError_t mlp_predict_rows(const MlpArgs& a, cudaStream_t st);
 cudaError_t mlp_train_step(const MlpArgs& a, cudaStream_t st);
 

@@ -107,6 +107,7 @@ def lib():
         "pticm_smem_copy_rate": [C.c_int, P],
         "pticm_set_wait_limit": [P, u64, u32],
         "pticm_philox_probe": [P, P, P, C.c_int],
+        "pticm_mlp_division_probe": [P, P, P, C.c_int],
         "pticm_set_profiling": [P, C.c_int],
         "pticm_cae_ladder": [P, u64, dbl, dbl, C.c_int, u32, dbl, dbl, dbl, u64, u64, P, P],
         "pticm_enable_energy_histograms": [P, u64],
