@@ -782,7 +782,8 @@ def run_gpu_ladder(args):
         ttt.append(res)
         log(json.dumps(res))
     clk.__exit__(None, None, None)
-    # the network's GEMM on the tensor cores at an inference-sized shape
+    # the library's stand-alone GEMM on the tensor cores at the shape of one
+    # layer (the network itself runs fused kernels, mlp_chain_kernel)
     import ctypes as C
     L = pticm.lib()
     L.pticm_tc_gemm_bench.argtypes = [C.c_int, C.c_int, C.c_int, C.c_int, C.c_void_p, C.c_void_p]
@@ -826,7 +827,8 @@ def run_gpu_ladder(args):
         "roofline": {"bound": "tensor", "kernel": "tc_gemm_tma_kernel (TMA loads, tcgen05 MMA, BF16, FP32 accumulate)",
                      "achieved": gemm.get("65536x256x256", {}).get("tflops"), "peak": bf16_peak, "unit": "TFLOP/s",
                      "frac": (gemm.get("65536x256x256", {}).get("tflops") or 0.0) / bf16_peak,
-                     "note": f"one 256x256 layer of the network on 65536 rows; peak {peak_kind} cuBLAS bf16",
+                     "note": "the stand-alone GEMM at the shape of one 256x256 layer on 65536 rows, not the network's "
+                             f"own fused kernel (mlp_chain_kernel); peak {peak_kind} cuBLAS bf16",
                      "shapes": gemm},
     }
     print(json.dumps(line), flush=True)
