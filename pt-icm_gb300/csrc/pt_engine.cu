@@ -2173,7 +2173,7 @@ static __device__ void exchange_replay(const EngineArgs& A, const BlockCtx& B, i
 
 // ---------------------------------------------------------------- kernel
 // Launch bounds: blocks of several replicas, and narrow block teams (NARROW),
-// run at most kNarrowThreads threads, which leaves each thread 120 registers
+// run at most kNarrowThreads threads, which leaves each thread 128 registers
 // instead of the 64 of a 1024-thread bound; replay and wide block teams (one
 // replica of a large instance per block) keep 1024.
 template <bool REPLAY, bool BLOCKTEAM, bool NARROW, int SPACE>

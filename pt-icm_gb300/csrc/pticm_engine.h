@@ -197,7 +197,7 @@ enum EngineFlags : int32_t {
 // Shared-memory scratch of one ICM team for an instance of n_pad sites: BFS
 // queue / labels (4 B per site), overlap flags (1 B per site), visited bits.
 // Threads of a block of several replicas, or of a block team launched with
-// the narrow bound (120 registers a thread).
+// the narrow bound (at most 128 registers a thread).
 constexpr int kNarrowThreads = 512;
 // Published energy words (flag_barrier) sit one per 128-byte line, so that
 // the blocks polling a group's words do not all queue on a few lines:

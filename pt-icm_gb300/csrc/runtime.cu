@@ -266,7 +266,7 @@ int choose_config(const HostProblem& P, const pticm_opts& o, bool replay, Instan
     if (threads <= 0) {
         // several replicas per block: the 512-thread bound; one replica per
         // block: at most the narrow-bound block (on N=2000, 512 threads at
-        // 120 registers beat 1024 threads at 64 by 11 %)
+        // up to 128 registers beat 1024 threads at 64 by 11 %)
         if (rpc > 1) threads = kNarrowThreads;
         else threads = std::min(kNarrowThreads, std::max(128, ((std::max(max_class, n / 2) + 31) / 32) * 32));
     }

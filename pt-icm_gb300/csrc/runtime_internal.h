@@ -65,7 +65,7 @@ inline int32_t pad16(int64_t n) { return (int32_t)((n + 15) & ~15ll); }
 struct LaunchConfig {
     int rpc = 0, group = 0, threads = 0, teams = 1;
     bool block_team = false;
-    bool narrow = false;         // block team on the narrow-bound kernel (kNarrowThreads, 120 registers)
+    bool narrow = false;         // block team on the narrow-bound kernel (kNarrowThreads, at most 128 registers)
     bool state_global = false;   // replica state and ICM scratch in device memory
     bool field_gather = false;   // spins in shared memory, fields gathered at each visit
     SmemPlan plan{};
