@@ -209,7 +209,7 @@ int pticm_mlp_create(uint64_t seed, uint32_t batch, pticm_mlp** out) {
     bad |= m->alloc(&A.Vm, kParams) != cudaSuccess;
     for (int l = 0; l < MLP_LAYERS; l++) {
         bad |= m->alloc(&A.Wi[l], (size_t)MLP_H * kKin[l] * 2) != cudaSuccess;
-        bad |= m->alloc(&A.WTi[l], (size_t)MLP_H * kKin[l] * 2) != cudaSuccess;
+        if (l > 0) bad |= m->alloc(&A.WTi[l], (size_t)MLP_H * kKin[l] * 2) != cudaSuccess;
         bad |= m->alloc(&A.Z[l], B * MLP_H / 4) != cudaSuccess;
         bad |= m->alloc(&A.dZf[l], B * MLP_H / 4) != cudaSuccess;
         bad |= m->alloc(&A.dZT[l], B * MLP_H * 2) != cudaSuccess;

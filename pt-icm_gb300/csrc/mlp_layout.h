@@ -30,7 +30,6 @@ constexpr size_t kParams = kB5 + 1;
 // u ^ (r & 7)).  A tile's chunk is one contiguous bulk copy.
 constexpr uint32_t kChunkRow = 128;                          // bytes of a row in a chunk
 constexpr uint32_t kChunkH = MLP_H * kChunkRow;              // a chunk of a 256-row matrix: 32 KB
-constexpr uint32_t kChunkIn = MLP_K0 * kChunkRow;            // of a 64-row matrix: 8 KB
 
 // Byte of element (row r, column k) in an image of `rows` rows.
 __host__ __device__ constexpr size_t image_at(int r, long long k, int rows) {
@@ -54,7 +53,7 @@ struct MlpArgs {
     float* G;
     float* Mm;
     float* Vm;
-    uint8_t* Wi[MLP_LAYERS];   // images of W_l [256 x K_l] and of W_l^T [K_l x 256] (bf16)
+    uint8_t* Wi[MLP_LAYERS];   // images of W_l [256 x K_l] and, but for the first layer, of W_l^T [K_l x 256] (bf16)
     uint8_t* WTi[MLP_LAYERS];
     float4* Z[MLP_LAYERS];     // pre-activations, tiled
     float4* dZf[MLP_LAYERS];   // their gradients, tiled

@@ -71,35 +71,6 @@ __device__ __forceinline__ uint2 stream_key(unsigned long long seed, uint32_t ta
     return make_uint2((uint32_t)seed ^ tag, (uint32_t)(seed >> 32) ^ (tag * 0x9E3779B9u));
 }
 
-// A per-thread buffered Philox stream: four 32-bit words per block call.
-struct ThreadRng {
-    uint4 buf;
-    uint32_t avail;
-    uint32_t calls;
-    uint4 ctr;   // (thread id, step lo, step hi, call index)
-    uint2 key;
-
-    __device__ __forceinline__ void start(uint2 k, uint32_t tid, unsigned long long step) {
-        key = k;
-        ctr = make_uint4(tid, (uint32_t)step, (uint32_t)(step >> 32), 0u);
-        avail = 0;
-        calls = 0;
-    }
-    __device__ __forceinline__ uint32_t next() {
-        if (avail == 0) {
-            ctr.w = calls++;
-            buf = philox4x32_10(ctr, key);
-            avail = 4;
-        }
-        const uint32_t r = buf.x;
-        buf.x = buf.y;
-        buf.y = buf.z;
-        buf.z = buf.w;
-        avail--;
-        return r;
-    }
-};
-
 // Three Philox blocks with interleaved rounds (independent chains overlap).
 __device__ __forceinline__ void philox4x32_10_x3(uint4& a, uint4& b, uint4& c, uint2 k) {
 #pragma unroll
