@@ -205,6 +205,12 @@ PTICM_API int pticm_get_exchange_order(pticm_ctx* c, uint32_t* order);
  * src/mpi_utils.cc:223-225 assert or exit). */
 PTICM_API int pticm_set_wait_limit(pticm_ctx* c, uint64_t limit_ns, uint32_t phantom_arrivals);
 
+/* Test hook: every second block holds its published spins back for delay_ns
+ * (at most 100 ms; 0: none) after its energies, so that the blocks of its
+ * replicas' partners meet words of an earlier step and have to wait for the
+ * step's. */
+PTICM_API int pticm_set_publish_delay(pticm_ctx* c, uint32_t delay_ns);
+
 /* The engine layout a context runs (chosen at pticm_init_states /
  * pticm_set_states): replicas per block, blocks, threads per block, ICM teams
  * per block (1: the whole block is one team), whether one block holds one

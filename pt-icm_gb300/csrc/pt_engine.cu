@@ -2467,6 +2467,10 @@ __global__ void __launch_bounds__((REPLAY || (BLOCKTEAM && !NARROW)) ? 1024 : kN
                 if (observe) st_release_gpu_u64(ew + (B.r0 + j) * kPubStride, w);
                 else st_relaxed_gpu_u64(ew + (B.r0 + j) * kPubStride, w);
             }
+            if (A.publish_delay_ns && (B.rank & 1)) {
+                const unsigned long long from = globaltimer_ns();
+                while (globaltimer_ns() - from < A.publish_delay_ns) __nanosleep(200);
+            }
             if (icm_on) publish_spins();
             draw();
             const unsigned long long limit = A.wait_limit_ns ? A.wait_limit_ns : kWaitLimitNs;

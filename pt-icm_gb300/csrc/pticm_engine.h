@@ -181,6 +181,10 @@ struct EngineArgs {
     // every energy lies in (-2^30, 2^30): energy changes and sums are exact
     // modulo 2^32
     int32_t small_energy;
+    // every second block holds its spin words back this long after its energy
+    // words (0 in production; a test hook that makes partners meet words of an
+    // earlier step)
+    uint32_t publish_delay_ns;
 };
 
 enum EngineFlags : int32_t {

@@ -125,6 +125,7 @@ struct pticm_ctx {
     // bounded waits: limit (0 = kWaitLimitNs) and the barrier test hook
     unsigned long long wait_limit_ns = 0;
     int bar_phantom = 0;
+    uint32_t publish_delay_ns = 0;
     // the inputs of the last launch configuration (it depends on nothing else
     // once the context exists): replay, ICM pairs, histogram rows
     bool configured = false;
@@ -691,6 +692,7 @@ EngineArgs make_args(pticm_ctx* c) {
     A.icm_pub_stride = c->icm_pub_stride;
     A.wait_limit_ns = c->wait_limit_ns;
     A.bar_phantom = c->bar_phantom;
+    A.publish_delay_ns = c->publish_delay_ns;
     if (c->ebound < 0) c->ebound = energy_bound(c->P);
     A.flag_barrier = c->ebound < (1ll << 31) ? 1 : 0;   // every energy fits the word's 32 bits
     A.small_energy = c->ebound < (1ll << 30) ? 1 : 0;
@@ -1315,6 +1317,13 @@ int pticm_set_wait_limit(pticm_ctx* c, uint64_t limit_ns, uint32_t phantom_arriv
     if (phantom_arrivals > 1) return fail(PTICM_ERR_INVALID, "phantom_arrivals must be 0 or 1");
     c->wait_limit_ns = limit_ns;
     c->bar_phantom = (int)phantom_arrivals;
+    return PTICM_OK;
+}
+
+int pticm_set_publish_delay(pticm_ctx* c, uint32_t delay_ns) {
+    if (!c) return fail(PTICM_ERR_INVALID, "null argument");
+    if (delay_ns > 100000000u) return fail(PTICM_ERR_INVALID, "publish delay above 100 ms");
+    c->publish_delay_ns = delay_ns;
     return PTICM_OK;
 }
 

@@ -106,6 +106,7 @@ def lib():
         "pticm_get_paths": [P, P, P],
         "pticm_smem_copy_rate": [C.c_int, P],
         "pticm_set_wait_limit": [P, u64, u32],
+        "pticm_set_publish_delay": [P, u32],
         "pticm_philox_probe": [P, P, P, C.c_int],
         "pticm_mlp_division_probe": [P, P, P, C.c_int],
         "pticm_set_profiling": [P, C.c_int],
@@ -396,6 +397,10 @@ class Context:
         """Limit of every wait on other blocks (0: 2 s); phantom_arrivals=1
         makes every group barrier wait for a block that never comes."""
         _check(lib().pticm_set_wait_limit(self._h, int(limit_ns), int(phantom_arrivals)))
+
+    def set_publish_delay(self, delay_ns=0):
+        """Test hook: every second block holds its published spins back this long."""
+        _check(lib().pticm_set_publish_delay(self._h, int(delay_ns)))
 
     def set_profiling(self, enable=True):
         _check(lib().pticm_set_profiling(self._h, int(enable)))
