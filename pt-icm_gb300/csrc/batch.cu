@@ -268,7 +268,7 @@ int configure_batch(pticm_batch* b) {
     BCK(b->d_desc.upload(b->desc));
     BCK(b->d_sched_off.upload(b->sched_off));
     BCK(b->d_sched.upload(b->sched));
-    BCK(default_stream_done());
+    BCK(after_default_stream(b->stream));
     return PTICM_OK;
 }
 
@@ -521,7 +521,7 @@ int pticm_batch_create(const pticm_problem* const* problems, uint32_t count, con
     BCK(b->d_abort.alloc(1));
     BCK(b->d_status.alloc(1));
     BCK(b->d_mismatch.alloc(1));
-    BCK(default_stream_done());
+    BCK(after_default_stream(b->stream));
     // smallest group per instance: replicas of a block fit shared memory
     // (unstaged, one ICM team) on their own
     b->gmin.assign(count, 0);
@@ -570,7 +570,7 @@ int pticm_batch_set_ladders(pticm_batch* b, const double* beta, uint32_t nt, int
     }
     BCK(b->d_beta.upload(b->beta));
     BCK(b->d_thr.upload(thr_all, 4));
-    BCK(default_stream_done());
+    BCK(after_default_stream(b->stream));
     b->ladder_set = true;
     return PTICM_OK;
 }
@@ -645,7 +645,7 @@ int pticm_batch_autotune(pticm_batch* b, uint32_t trial_steps) {
         }
         DArr<unsigned long long> job_ns;
         BCK(job_ns.alloc(b->sched.size() / 2));
-        BCK(default_stream_done());
+        BCK(after_default_stream(b->stream));
         // a two-step launch sizes the trial so that it stays near the launch target
         float ms = 0.f;
         if (int rc = batch_launch(b, b->steps_done, 2, PHASE_SWEEP | PHASE_EXCHANGE | PHASE_ICM, nullptr, &ms))
@@ -832,7 +832,7 @@ int pticm_batch_enable_energy_histograms(pticm_batch* b, uint64_t from_step) {
     }
     if ((uint64_t)off > (1ull << 34)) return bfail(PTICM_ERR_UNSUPPORTED, "energy histograms of the batch exceed 64 GB");
     BCK(b->d_hist.alloc((size_t)off));
-    BCK(default_stream_done());
+    BCK(after_default_stream(b->stream));
     b->hist_from = from_step;
     b->hist_on = true;
     return PTICM_OK;

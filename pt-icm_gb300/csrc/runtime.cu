@@ -633,7 +633,7 @@ int configure(pticm_ctx* c, bool replay) {
     CK(c->d_sched_off.upload(soff));
     CK(c->d_sched.upload(sched));
     CK(c->d_desc.upload(std::vector<InstanceDesc>{c->desc}));
-    CK(default_stream_done());
+    CK(after_default_stream(c->stream));
     c->configured = true;
     c->cfg_replay = replay;
     c->cfg_nc = c->desc.nc;
@@ -1169,7 +1169,7 @@ int pticm_create(const pticm_problem* p, const pticm_opts* o, pticm_ctx** out) {
     std::vector<int32_t> ri(c->R, 0);
     CK(c->d_rep_inst.upload(ri));
     CK(c->d_desc.upload(std::vector<InstanceDesc>{D}));
-    CK(default_stream_done());
+    CK(after_default_stream(c->stream));
     *out = c.release();
     return PTICM_OK;
 }
@@ -1189,7 +1189,7 @@ int pticm_set_ladder(pticm_ctx* c, const double* beta, uint32_t nt, int32_t nc) 
     CK(c->d_beta.upload(c->beta));
     CK(c->d_thr.upload(thr, 4));
     CK(c->d_ptab.upload(ptab, 4));
-    CK(default_stream_done());
+    CK(after_default_stream(c->stream));
     c->ladder_set = true;
     return PTICM_OK;
 }
@@ -1260,7 +1260,7 @@ int pticm_icm_pairs(pticm_ctx* c, const int64_t* seeds, uint32_t count, int exac
     if (int rc = configure(c, false)) return rc;
     std::vector<long long> f(seeds, seeds + count);
     CK(c->d_icm_force.upload(f));
-    CK(default_stream_done());
+    CK(after_default_stream(c->stream));
     if (int rc = reset_flags(c)) return rc;
     EngineArgs A = make_args(c);
     A.step0 = c->steps_done;
@@ -1355,7 +1355,7 @@ int pticm_replay(pticm_ctx* c, const pticm_trace* t) {
     CK(d_xs.upload(xs, 1));
     CK(d_logu.upload(xl, 1));
     CK(d_seed.upload(seeds, 1));
-    CK(default_stream_done());
+    CK(after_default_stream(c->stream));
     if (int rc = reset_flags(c)) return rc;
     EngineArgs A = make_args(c);
     A.step0 = c->steps_done;
@@ -1497,7 +1497,7 @@ int pticm_set_profiling(pticm_ctx* c, int enable) {
     if (!c) return fail(PTICM_ERR_INVALID, "null argument");
     c->profiling = enable != 0;
     if (c->profiling) CK(c->d_prof.alloc((size_t)std::max(c->R, 1) * PROF_PHASES));
-    CK(default_stream_done());
+    CK(after_default_stream(c->stream));
     return PTICM_OK;
 }
 
@@ -1543,7 +1543,7 @@ int pticm_enable_energy_histograms(pticm_ctx* c, uint64_t from_step) {
     CK(c->d_hist.alloc((size_t)c->R * (size_t)c->hist_nbins));
     CK(c->d_obs.alloc(2 * (size_t)c->R));
     CK(c->d_mag_pub.alloc(2 * (size_t)c->R));
-    CK(default_stream_done());
+    CK(after_default_stream(c->stream));
     return PTICM_OK;
 }
 
@@ -1852,7 +1852,7 @@ int pticm_checkpoint_load(pticm_ctx* c, const char* path) {
     if (!rc && hist_nbins > 0) rc = ckpt_restore(F, c->d_hist, "histograms");
     if (!rc && hist_nbins > 0) rc = ckpt_restore(F, c->d_obs, "observables");
     if (rc) return rc;
-    CK(default_stream_done());
+    CK(after_default_stream(c->stream));
     c->steps_done = steps;
     c->attempts = attempts;
     c->states_set = true;

@@ -17,8 +17,16 @@ constexpr long long kNoBest = std::numeric_limits<long long>::max();
 
 // The runtime's streams do not wait for the default stream, on which DArr
 // clears and fills its buffers (a clear, or a copy from pageable memory, may
-// return before it has landed): called before such buffers are used on them.
-inline cudaError_t default_stream_done() { return cudaStreamSynchronize(cudaStreamLegacy); }
+// return before it has landed): called before such buffers are used on `st`.
+inline cudaError_t after_default_stream(cudaStream_t st) {
+    cudaEvent_t ev = nullptr;
+    cudaError_t e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
+    if (e != cudaSuccess) return e;
+    e = cudaEventRecord(ev, cudaStreamLegacy);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(st, ev, 0);
+    cudaEventDestroy(ev);   // (its resources go when the wait is over)
+    return e;
+}
 
 template <typename T>
 struct DArr {
