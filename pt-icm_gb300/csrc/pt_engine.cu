@@ -110,7 +110,9 @@ enum TeamCtl : int {
     TC_S = 4,         // sites listed outside the giant component, zero between pairs
     TC_STALE = 5,     // a published word had not arrived, zero between pairs
     TC_COUNT = 6,     // a sum of counts; zeroed when a pair begins
+    TC_EXPIRED = 7,   // the wait for published words ran out
     TC_DE = 8,        // two 64-bit energy changes; zeroed when a pair begins
+    TC_DEADLINE = 12, // 64-bit time at which that wait ends (a warp team's lies in its two words)
     TC_WORDS = 16
 };
 
@@ -509,12 +511,27 @@ __device__ __forceinline__ int icm_pair(const EngineArgs& A, const BlockCtx& B, 
     if (!again) break;
     // a partner's word had not arrived (its block published it before the
     // energy this block waited for, but nothing orders the two): once more,
-    // at most as long as any wait on another block (a pass takes over 500 ns)
-    const unsigned long long limit = A.wait_limit_ns ? A.wait_limit_ns : kWaitLimitNs;
+    // at most as long as any wait on another block, and not when another has
+    // ended the run (the deadline lies in shared memory: the passes before it
+    // is needed keep no register for it)
     team.sync();
-    if (BLOCK && team.tr == 0) { team.ctl[TC_OVERLAP] = 0; team.ctl[TC_OTHERS] = 0; team.ctl[TC_STALE] = 0; }
+    int expired = 0;
+    if (team.tr == 0) {
+        volatile unsigned long long* const deadline =
+            reinterpret_cast<unsigned long long*>(team.ctl + (BLOCK ? TC_DEADLINE : TC_BEST));
+        const unsigned long long t = globaltimer_ns();
+        if (tries == 0) *deadline = t + (A.wait_limit_ns ? A.wait_limit_ns : kWaitLimitNs);
+        else expired = t > *deadline || *(volatile int*)A.abort_flag != 0;
+        if (BLOCK) {
+            team.ctl[TC_OVERLAP] = 0;
+            team.ctl[TC_OTHERS] = 0;
+            team.ctl[TC_STALE] = 0;
+            team.ctl[TC_EXPIRED] = expired;
+        }
+    }
     team.sync();
-    if (tries > limit / 500) {
+    expired = BLOCK ? *(volatile int*)(team.ctl + TC_EXPIRED) : __shfl_sync(0xffffffffu, expired, 0);
+    if (expired) {
         // (the run ends with this error at the group's next meeting)
         if (team.tr == 0) dev_fail(A.status, A.abort_flag, DEV_BARRIER_TIMEOUT, 4, blockIdx.x, tag);
         return 0;

@@ -76,3 +76,15 @@ def test_words_that_stay_away_end_the_run(name):
     ctx.set_publish_delay(0)
     ctx.run(5)
     assert ctx.verify() == 0
+
+
+def test_the_limit_holds_where_a_pass_is_long():
+    """A pass over 40000 sites takes tens of microseconds: the wait still ends at its limit, long before the words come."""
+    import pticm
+    ctx = _context(40000, 6, replicas_per_block=4, icm_algo=1)
+    ctx.run(2)
+    ctx.set_wait_limit(limit_ns=2_000_000)
+    ctx.set_publish_delay(40_000_000)
+    with pytest.raises(pticm.PticmError) as e:
+        ctx.run(1)
+    assert e.value.code == 5 and "wait expired at site 4" in str(e.value)
