@@ -1271,9 +1271,10 @@ __device__ __forceinline__ int gather_pieces(const int32_t* row, const uint32_t*
 // replicas: tagged words of the sites to flip and the new energies, eight
 // sites per thread and replica, four replicas' words loaded together.  (Every
 // block has published its results or is working on them: no block waits
-// before its own pairs are out.)
+// before its own pairs are out.)  False in a warp whose wait ran out: replicas
+// may then be flipped in part, and no sweep may follow.
 template <int SPACE>
-__device__ __forceinline__ void apply_pairs(const EngineArgs& A, const BlockCtx& B, int chains_even, uint32_t tag,
+__device__ __forceinline__ bool apply_pairs(const EngineArgs& A, const BlockCtx& B, int chains_even, uint32_t tag,
                                             volatile int* abortf) {
     const InstanceDesc& D = B.D;
     const int tid = threadIdx.x, T = blockDim.x, n = D.n, nt = D.nt, W = (n + 31) >> 5;
@@ -1294,7 +1295,7 @@ __device__ __forceinline__ void apply_pairs(const EngineArgs& A, const BlockCtx&
             if (from[x] != nullptr) {
                 if (tid < 32) {
                     unsigned long long w = 0;
-                    if (!poll_tagged(from[x] + 2 * W + second, tid == 0, tag, w, abortf, A.status, limit, 6)) return;
+                    if (!poll_tagged(from[x] + 2 * W + second, tid == 0, tag, w, abortf, A.status, limit, 6)) return false;
                     if (tid == 0) B.E[B.r0 + j0 + x] = (long long)(int32_t)(uint32_t)w;
                 }
                 if (second) from[x] += W;
@@ -1312,7 +1313,7 @@ __device__ __forceinline__ void apply_pairs(const EngineArgs& A, const BlockCtx&
                 const bool late = u < 4 * W && (uint32_t)(w[x] >> 32) != tag;
                 if (__any_sync(0xffffffffu, late) &&
                     !poll_tagged(from[x] + (late ? u >> 2 : 0), late, tag, w[x], abortf, A.status, limit, 6))
-                    return;
+                    return false;
                 const SpinRow<SPACE> sp = spin_row<SPACE>(B, j0 + x);
                 for (uint32_t m = ((uint32_t)w[x] >> (8 * (u & 3))) & 0xffu; m != 0 && u < 4 * W; m &= m - 1) {
                     const int i = 8 * u + __ffs((int)m) - 1;
@@ -1321,6 +1322,7 @@ __device__ __forceinline__ void apply_pairs(const EngineArgs& A, const BlockCtx&
             }
         }
     }
+    return true;
 }
 
 // The local fields of four interleaved replicas at one site per lane (its list
@@ -2605,7 +2607,7 @@ __global__ void __launch_bounds__((REPLAY || (BLOCKTEAM && !NARROW)) ? 1024 : kN
                 }
                 if (share) {
                     __syncthreads();
-                    apply_pairs<SPACE>(A, B, chains_even, A.pub_base + (uint32_t)ls, abortf);
+                    if (!__syncthreads_and(apply_pairs<SPACE>(A, B, chains_even, A.pub_base + (uint32_t)ls, abortf))) break;
                 }
             } else {
                 const int warp = tid >> 5, lane = tid & 31;

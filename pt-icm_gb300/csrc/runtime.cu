@@ -1238,7 +1238,16 @@ int pticm_run(pticm_ctx* c, uint64_t pt_steps, uint32_t phase_mask) {
         float ms = 0.f;
         CK(cudaEventElapsedTime(&ms, c->ev0, c->ev1));
         c->last_ms += ms;
-        if (int rc = read_status(c, "pticm_run")) return rc;
+        if (int rc = read_status(c, "pticm_run")) {
+            // (a block that takes over other blocks' results may have flipped
+            // a replica in part when its wait ran out: the energies and
+            // fields of the spins as they are)
+            if (A.icm_pub) {
+                CK(launch_recompute(A, c->d_rep_inst.p, c->R, 1, nullptr, nullptr, nullptr, c->stream));
+                CK(cudaStreamSynchronize(c->stream));
+            }
+            return rc;
+        }
         c->steps_done += (uint64_t)chunk;
         if (phase_mask & PHASE_SWEEP) c->attempts += (uint64_t)chunk * c->o.sweeps * (uint64_t)c->R * (uint64_t)c->P.n;
         left -= (uint64_t)chunk;

@@ -36,8 +36,11 @@ LAYOUTS = {
     "warp_teams": (201, 6, dict(replicas_per_block=2)),
     "block_team_of_three": (900, 6, dict(replicas_per_block=3)),
     "spins_only": (60000, 6, dict(replicas_per_block=1)),
-    "shared_pairs": (45001, 6, dict(replicas_per_block=2)),
-    "interleaved": (40000, 6, dict(replicas_per_block=4)),
+    "scratch_in_device_memory_2": (45001, 6, dict(replicas_per_block=2)),
+    "scratch_in_device_memory_4": (40000, 6, dict(replicas_per_block=4)),
+    # (the cluster search's scratch fits beside the spins: every pair is worked out once)
+    "shared_pairs": (20001, 6, dict(replicas_per_block=2)),
+    "shared_pairs_interleaved": (14016, 6, dict(replicas_per_block=4)),
 }
 
 
@@ -88,3 +91,22 @@ def test_the_limit_holds_where_a_pass_is_long():
     with pytest.raises(pticm.PticmError) as e:
         ctx.run(1)
     assert e.value.code == 5 and "wait expired at site 4" in str(e.value)
+
+
+def test_a_run_that_ends_between_shared_pairs_leaves_exact_energies():
+    """With pairs worked out once, a block may have taken over some of its replicas' results when another's never comes."""
+    import pticm
+    ctx = _context(14016, 6, replicas_per_block=4)
+    ctx.set_ladder(pticm.beta_linspace(1.0, 1.01, NT), nc=NT)   # (close enough that replicas change places in every step)
+    for trial in range(30):
+        ctx.run(5)
+        ctx.set_wait_limit(limit_ns=1_000_000)
+        ctx.set_publish_delay(10_000_000)
+        with pytest.raises(pticm.PticmError) as e:
+            ctx.run(4)
+        assert e.value.code == 5 and "wait expired" in str(e.value)
+        assert ctx.verify() == 0, trial
+        E, _, state, _ = ctx.best()
+        assert ctx.problem.evaluate(state[None, :])[0][0] == E, trial
+        ctx.set_wait_limit(0)
+        ctx.set_publish_delay(0)
